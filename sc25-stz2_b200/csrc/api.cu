@@ -5,8 +5,8 @@
 //      FD5:92-104);
 //   2. coarsest grid = field sampled every 2^K points (stored raw);
 //   3. one fused level-encode launch per level, coarse to fine (levels.cu);
-//   4. histogram windows to the host, canonical codebooks on the host pool;
-//   5. entropy coding on the GPU: code tables, plane bit counts, offsets scan
+//   4. canonical codebooks from the code histograms (codebook.cu);
+//   5. entropy coding on the GPU: plane bit counts, offsets scan
 //      (marker tables), encode, unpredictable-value gather, payload pack;
 //   6. per-layer zstd frames on the host pool and the container.
 // Decompress: zstd frames on the host pool into one pinned staging buffer, one
@@ -510,177 +510,173 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaGetLastError());
 
     std::vector<StreamDesc> sd = g.sd;
-    // work list over every chunk of every stream
+    cudaStream_t sc = ctx->st_copy;
+    struct Events {
+        std::vector<cudaEvent_t> e;
+        ~Events()
+        {
+            for (cudaEvent_t x : e) cudaEventDestroy(x);
+        }
+    } ev;
+    // Work lists over every chunk of every stream, in the groups the payload
+    // is encoded, packed and copied back in: every stream of the coarser
+    // levels, then the finest level's streams in two halves of their chunk
+    // z-layers (all 7 streams per group, so every launch still fills the
+    // device); the host zstd-compresses a group's frames while the device
+    // encodes the next (one, two, four or eight finest groups measured within
+    // noise of each other once payload frames skip zstd; two is the fewest
+    // launches that still overlap the copy back).
+    const int fin0 = std::max(0, nstreams - 7);
+    const int fin_layers = (int)sd[nstreams - 1].ncz;
+    const int lpg = std::max(1, (fin_layers + 1) / 2);  // layers per group: two finest groups
+    const size_t ngroups = 1 + (size_t)((fin_layers + lpg - 1) / lpg);
     std::vector<CtaWork> work;
     std::vector<uint32_t> ids;
-    for (int s = 0; s < nstreams; ++s) add_all_chunks(work, ids, (uint32_t)s, sd[s].nchunks, (int)sd[s].C);
-    // Run statistics of every stream whose planes can take run symbols: one
-    // pass over the codes right after the level encodes, while the histograms
-    // go to the host. The counts per run class depend only on the plane size
-    // and the codes, not on which free code values the stream's run symbols
-    // later take; here they are numbered from R2, above every code, so no
-    // literal is taken for one. Work list and counters go up on the copy
-    // stream while the device runs the levels.
-    std::vector<unsigned long long> rstats((size_t)nstreams * kRunStats, 0);
+    std::vector<size_t> gw(ngroups + 1, 0);
+    for (int s = 0; s < fin0; ++s) add_all_chunks(work, ids, (uint32_t)s, sd[s].nchunks, (int)sd[s].C);
+    for (size_t gi = 1; gi < ngroups; ++gi) {
+        gw[gi] = work.size();
+        const int L0 = (int)(gi - 1) * lpg, L1 = std::min(fin_layers, L0 + lpg);
+        for (int s = fin0; s < nstreams; ++s) {
+            const uint32_t cpl = sd[s].ncx * sd[s].ncy;
+            std::vector<uint32_t> cs;
+            for (uint32_t c = (uint32_t)L0 * cpl; c < (uint32_t)L1 * cpl; ++c) cs.push_back(c);
+            add_work(work, ids, (uint32_t)s, cs.data(), cs.size(), (int)sd[s].C);
+        }
+    }
+    gw[ngroups] = work.size();
+    // The run symbols of every stream whose planes can take them are counted
+    // in one pass over the codes. The counts per run class depend only on the
+    // plane size and the codes, not on which free code values the stream's
+    // run symbols later take; here they are numbered from R2, above every
+    // code, so no literal is taken for one. The codebook kernels then put the
+    // stream's own values into the descriptors. Descriptors, work lists and
+    // counters go up on the copy stream while the device runs the levels.
     bool rs_any = false;
-    size_t r_sd = 0, r_work = 0, r_ids = 0;
-    cudaEvent_t ev_up = ctx->event();
-    {
-        std::vector<StreamDesc> rsd = sd;
-        for (auto& d : rsd) {
-            d.run_n = run_slot_count(d.C * d.C);
-            d.run_base = (uint32_t)R2;
-            rs_any = rs_any || d.run_n;
-        }
-        if (rs_any) {
-            r_work = align256(rsd.size() * sizeof(StreamDesc));
-            r_ids = align256(r_work + work.size() * sizeof(CtaWork));
-            const size_t r_bytes = align256(r_ids + ids.size() * 4);
-            STZ_CUDA(ctx->h_stage.ensure(r_bytes));
-            uint8_t* hr = ctx->h_stage.as<uint8_t>();
-            std::memcpy(hr + r_sd, rsd.data(), rsd.size() * sizeof(StreamDesc));
-            std::memcpy(hr + r_work, work.data(), work.size() * sizeof(CtaWork));
-            std::memcpy(hr + r_ids, ids.data(), ids.size() * 4);
-            STZ_CUDA(ctx->work.ensure(r_bytes));
-            STZ_CUDA(cudaMemcpyAsync(ctx->work.p, hr, r_bytes, cudaMemcpyHostToDevice, ctx->st_copy));
-            STZ_CUDA(ctx->rstats.ensure(rstats.size() * 8));
-            STZ_CUDA(cudaMemsetAsync(ctx->rstats.p, 0, rstats.size() * 8, ctx->st_copy));
-            STZ_CUDA(ctx->h_rstats.ensure(rstats.size() * 8));
-            STZ_CUDA(cudaEventRecord(ev_up, ctx->st_copy));
-        }
+    std::vector<uint64_t> cb_items(nstreams + 1, 0);
+    uint32_t max_chunks = 0;
+    for (int s = 0; s < nstreams; ++s) {
+        sd[s].run_n = run_slot_count(sd[s].C * sd[s].C);
+        sd[s].run_base = (uint32_t)R2;
+        rs_any = rs_any || sd[s].run_n;
+        cb_items[s + 1] = cb_items[s] + codebook_items(sd[s], g.lv[s / 7 + 1].n);
+        max_chunks = std::max(max_chunks, sd[s].nchunks);
     }
+    const uint64_t cb_cap = cb_items[nstreams];
+    // sd | work | ids | codebook scratch offsets
+    const size_t o_work = align256(sd.size() * sizeof(StreamDesc));
+    const size_t o_ids = align256(o_work + work.size() * sizeof(CtaWork));
+    const size_t o_cbi = align256(o_ids + ids.size() * 4), up_bytes = align256(o_cbi + cb_items.size() * 8);
+    STZ_CUDA(ctx->h_stage.ensure(up_bytes));
+    uint8_t* hs = ctx->h_stage.as<uint8_t>();
+    std::memcpy(hs, sd.data(), sd.size() * sizeof(StreamDesc));
+    std::memcpy(hs + o_work, work.data(), work.size() * sizeof(CtaWork));
+    std::memcpy(hs + o_ids, ids.data(), ids.size() * 4);
+    std::memcpy(hs + o_cbi, cb_items.data(), cb_items.size() * 8);
+    STZ_CUDA(ctx->sd.ensure(up_bytes));
+    STZ_CUDA(cudaMemcpyAsync(ctx->sd.p, hs, up_bytes, cudaMemcpyHostToDevice, sc));
+    STZ_CUDA(ctx->rstats.ensure((size_t)nstreams * kRunStats * 8));
+    STZ_CUDA(cudaMemsetAsync(ctx->rstats.p, 0, (size_t)nstreams * kRunStats * 8, sc));
+    uint8_t* dstage = ctx->sd.as<uint8_t>();
+    StreamDesc* d_sd = (StreamDesc*)dstage;
+    const CtaWork* d_work = (const CtaWork*)(dstage + o_work);
+    const uint32_t* d_ids = (const uint32_t*)(dstage + o_ids);
+    const uint64_t* d_cbi = (const uint64_t*)(dstage + o_cbi);
 
-    // histogram windows + outside counts + unpred counts to the host, on the
-    // copy stream, while ctx->st counts the run symbols
-    const int wlo = std::max(0, o.radius - kHistWindow / 2);
-    const int wn = std::min(kHistWindow, R2 - wlo);
-    STZ_CUDA(ctx->h_hist.ensure((size_t)nstreams * wn * 4));
-    const size_t meta_bytes = (size_t)nstreams * 4 + g.total_chunk_slots * 4;
-    STZ_CUDA(ctx->h_meta.ensure(meta_bytes));
-    cudaStream_t sc = ctx->st_copy;
-    cudaEvent_t ev_lv = ctx->event(), ev_hist = ctx->event();
-    STZ_CUDA(cudaEventRecord(ev_lv, st));
-    STZ_CUDA(cudaStreamWaitEvent(sc, ev_lv, 0));
-    STZ_CUDA(cudaMemcpy2DAsync(ctx->h_hist.p, (size_t)wn * 4, ctx->hist.as<uint32_t>() + wlo, (size_t)R2 * 4,
-                               (size_t)wn * 4, (size_t)nstreams, cudaMemcpyDeviceToHost, sc));
-    uint32_t* h_out = ctx->h_meta.as<uint32_t>();
-    uint32_t* h_ucnt = h_out + nstreams;
-    STZ_CUDA(cudaMemcpyAsync(h_out, ctx->hist_out.p, (size_t)nstreams * 4, cudaMemcpyDeviceToHost, sc));
-    STZ_CUDA(cudaMemcpyAsync(h_ucnt, ctx->unpred_cnt.p, g.total_chunk_slots * 4, cudaMemcpyDeviceToHost, sc));
-    STZ_CUDA(cudaEventRecord(ev_hist, sc));
+    // codebook lists (info | symbols | lengths) and the coder's tables
+    const size_t o_sym = align256((size_t)nstreams * sizeof(CodebookInfo)), o_len = align256(o_sym + cb_cap * 2);
+    STZ_CUDA(ctx->books.ensure(o_len + cb_cap));
+    STZ_CUDA(ctx->cb_scratch.ensure(codebook_scratch_bytes(cb_cap, nstreams)));
+    STZ_CUDA(ctx->ctab.ensure((size_t)nstreams * R2 * 4));
+    STZ_CUDA(ctx->rbits.ensure((size_t)nstreams * kRunBitsStride));
+    STZ_CUDA(ctx->sub_bits.ensure(g.total_sub * 4));
+    STZ_CUDA(ctx->sub_off.ensure(g.total_sub * 4));
+    STZ_CUDA(ctx->chunk_off.ensure(g.total_chunk_slots * 8));
+    STZ_CUDA(ctx->stream_words.ensure((size_t)nstreams * 8 * 3));
+    STZ_CUDA(ctx->payload.ensure(g.total_words * 4));
+    // the coarser levels' streams (group 0) are many small ones: packed back
+    // to back on the device, they go to the host in one transfer
+    if (fin0 > 0) STZ_CUDA(ctx->packed.ensure(sd[fin0].word_base * 4));
+    uint8_t* dbooks = ctx->books.as<uint8_t>();
+    uint16_t* d_sym = (uint16_t*)(dbooks + o_sym);
+    uint8_t* d_len = dbooks + o_len;
+
+    // ev.e[gi]: group gi's words are on the host; ev.e[ngroups + gi]: its
+    // encode is done; then the named events below. The copies run on the
+    // context's copy stream, so group gi's copy overlaps group gi + 1's
+    // encode. The pool's threads wait on the copy events ev.e[0, ngroups)
+    // while others compress frames: those waits block instead of spinning on
+    // a core.
+    enum { EvUp, EvLevels, EvCounts, EvBooks, EvInfo, EvScan, EvTables, EvUnpred, EvNamed };
+    ev.e.assign(2 * ngroups + EvNamed, nullptr);
+    for (size_t i = 0; i < ev.e.size(); ++i)
+        STZ_CUDA(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming | (i < ngroups ? cudaEventBlockingSync : 0)));
+    cudaEvent_t* named = ev.e.data() + 2 * ngroups;
+    STZ_CUDA(cudaEventRecord(named[EvUp], sc));
+    STZ_CUDA(cudaEventRecord(named[EvLevels], st));
+    STZ_CUDA(cudaStreamWaitEvent(st, named[EvUp], 0));
+
+    // The rest of the device's work, from run symbols to payload words, goes
+    // out at once: nothing of it waits for the host.
     if (rs_any) {
-        STZ_CUDA(cudaStreamWaitEvent(st, ev_up, 0));
-        const uint8_t* dw = ctx->work.as<uint8_t>();
-        {
-            KScope ks(ctx, "k_run_stats");
-            launch_run_stats((const CtaWork*)(dw + r_work), (const uint32_t*)(dw + r_ids), (int)work.size(),
-                             (const StreamDesc*)(dw + r_sd), ctx->codes.as<uint16_t>(),
-                             ctx->rstats.as<unsigned long long>(), st);
-        }
-        STZ_CUDA(cudaGetLastError());
-        STZ_CUDA(cudaMemcpyAsync(ctx->h_rstats.p, ctx->rstats.p, rstats.size() * 8, cudaMemcpyDeviceToHost, st));
+        KScope ks(ctx, "k_run_stats");
+        launch_run_stats(d_work, d_ids, (int)work.size(), d_sd, ctx->codes.as<uint16_t>(),
+                         ctx->rstats.as<unsigned long long>(), st);
     }
     {
-        const cudaError_t e = cudaEventSynchronize(ev_hist);
-        ctx->ev_pool.push_back(ev_lv);
-        ctx->ev_pool.push_back(ev_hist);
-        ctx->ev_pool.push_back(ev_up);
-        STZ_CUDA(e);
+        KScope ks(ctx, "k_codebook", 2);
+        launch_codebooks(d_sd, nstreams, ctx->hist.as<uint32_t>(), ctx->hist_out.as<uint32_t>(),
+                         ctx->rstats.as<unsigned long long>(), d_cbi, cb_cap, ctx->cb_scratch.p,
+                         ctx->ctab.as<uint32_t>(), ctx->rbits.as<uint8_t>(), d_sym, d_len, (CodebookInfo*)dbooks, st);
     }
+    STZ_CUDA(cudaEventRecord(named[EvBooks], st));
+    {
+        KScope ks(ctx, "k_sub_bits");
+        launch_sub_bits(d_work, d_ids, (int)work.size(), d_sd, ctx->codes.as<uint16_t>(), ctx->ctab.as<uint32_t>(),
+                        ctx->rbits.as<uint8_t>(), ctx->sub_bits.as<uint32_t>(), st);
+    }
+    {
+        KScope ks(ctx, "k_scan_stream", 2);
+        launch_scan_streams(d_sd, nstreams, max_chunks, ctx->sub_bits.as<uint32_t>(), ctx->sub_off.as<uint32_t>(),
+                            ctx->chunk_off.as<uint64_t>(), ctx->stream_words.as<uint64_t>(),
+                            ctx->payload.as<uint32_t>(), st);
+    }
+    STZ_CUDA(cudaEventRecord(named[EvScan], st));
+    for (size_t gi = 0; gi < ngroups; ++gi) {
+        {
+            KScope ks(ctx, "k_encode");
+            launch_encode(d_work + gw[gi], d_ids, (int)(gw[gi + 1] - gw[gi]), d_sd, ctx->codes.as<uint16_t>(),
+                          ctx->ctab.as<uint32_t>(), ctx->rbits.as<uint8_t>(), ctx->sub_bits.as<uint32_t>(),
+                          ctx->sub_off.as<uint32_t>(), ctx->chunk_off.as<uint64_t>(), ctx->payload.as<uint32_t>(), st);
+        }
+        if (gi == 0 && fin0 > 0) {
+            KScope ks(ctx, "k_pack_streams");
+            launch_pack_streams(d_sd, ctx->stream_words.as<uint64_t>(), 0, fin0, ctx->payload.as<uint32_t>(),
+                                ctx->packed.as<uint32_t>(), st);
+        }
+        STZ_CUDA(cudaEventRecord(ev.e[ngroups + gi], st));
+    }
+    STZ_CUDA(cudaGetLastError());
+
+    // Unpredictable counts to the host after the levels (they size the value
+    // list), then what the headers need: codebooks, marker tables, plane
+    // offsets, values.
+    STZ_CUDA(ctx->h_meta.ensure(g.total_chunk_slots * 4));
+    uint32_t* h_ucnt = ctx->h_meta.as<uint32_t>();
+    STZ_CUDA(cudaStreamWaitEvent(sc, named[EvLevels], 0));
+    STZ_CUDA(cudaMemcpyAsync(h_ucnt, ctx->unpred_cnt.p, g.total_chunk_slots * 4, cudaMemcpyDeviceToHost, sc));
+    STZ_CUDA(cudaEventRecord(named[EvCounts], sc));
+    STZ_CUDA(ctx->h_hist.ensure(o_len + cb_cap));
+    uint8_t* hb = ctx->h_hist.as<uint8_t>();
+    STZ_CUDA(cudaStreamWaitEvent(sc, named[EvBooks], 0));
+    STZ_CUDA(cudaMemcpyAsync(hb, dbooks, (size_t)nstreams * sizeof(CodebookInfo), cudaMemcpyDeviceToHost, sc));
+    STZ_CUDA(cudaEventRecord(named[EvInfo], sc));
+    STZ_CUDA(cudaEventSynchronize(named[EvCounts]));
     std::vector<T> coarsest(n0);
     std::memcpy(coarsest.data(), ctx->h_small.as<uint8_t>() + 64, n0 * elem);
-    if (level_error_take()) STZ_FAIL(STZ_ERR_CUDA, "level kernel: a TMA tile load did not complete in time");
-    if (M && M->mask && learned_tc_error_take(st))
-        STZ_FAIL(STZ_ERR_CUDA, "learned correction: a tensor-core MMA did not complete in time");
-    lap.mark("levels + histograms");
+    lap.mark("levels");
 
-    // codebooks
-    std::vector<std::vector<uint16_t>> syms(nstreams);
-    std::vector<std::vector<uint8_t>> lens(nstreams);
-    // full histograms of the streams with codes outside the window: one
-    // pinned buffer, asynchronous copies, one wait
-    std::vector<const uint32_t*> fullh(nstreams, nullptr);
-    {
-        size_t nfull = 0;
-        for (int s = 0; s < nstreams; ++s) nfull += h_out[s] ? 1 : 0;
-        if (nfull) {
-            STZ_CUDA(ctx->h_fullh.ensure(nfull * (size_t)R2 * 4));
-            size_t k = 0;
-            for (int s = 0; s < nstreams; ++s)
-                if (h_out[s]) {
-                    uint32_t* dst = ctx->h_fullh.as<uint32_t>() + k++ * (size_t)R2;
-                    STZ_CUDA(cudaMemcpyAsync(dst, ctx->hist.as<uint32_t>() + (size_t)s * R2, (size_t)R2 * 4,
-                                             cudaMemcpyDeviceToHost, ctx->st_copy));
-                    fullh[s] = dst;
-                }
-            // on the copy stream: ctx->st is counting run symbols (the level
-            // encodes, all these copies need, are complete)
-            STZ_CUDA(cudaStreamSynchronize(ctx->st_copy));
-        }
-    }
-    lap.mark("full histograms");
-    // run symbols: J slots in unused code values, else none
-    for (int s = 0; s < nstreams; ++s) {
-        const uint32_t* hw = ctx->h_hist.as<uint32_t>() + s * (size_t)wn;
-        auto count = [&](uint32_t c) -> uint64_t {
-            if (h_out[s]) return (uint64_t)fullh[s][c];
-            return (c >= (uint32_t)wlo && c < (uint32_t)(wlo + wn)) ? hw[c - wlo] : 0;
-        };
-        sd[s].run_n = (uint32_t)run_slots(count, R2, (int)(sd[s].C * sd[s].C), sd[s].run_base);
-    }
-    lap.mark("run slots");
-    // the plain codebooks while the device counts the run symbols
-    ctx->pool->parallel_for((size_t)nstreams, [&](size_t s) {
-        const uint32_t* hw = h_out[s] ? fullh[s] : ctx->h_hist.as<uint32_t>() + s * (size_t)wn;
-        const int hn = h_out[s] ? R2 : wn, hb = h_out[s] ? 0 : wlo;
-        build_codebook(hw, hn, hb, syms[s], lens[s]);
-    });
-    lap.mark("plain codebooks");
-    if (rs_any) {
-        STZ_CUDA(cudaStreamSynchronize(st));
-        std::memcpy(rstats.data(), ctx->h_rstats.p, rstats.size() * 8);
-    }
-    lap.mark("run stats wait");
-    ctx->pool->parallel_for((size_t)nstreams, [&](size_t s) {
-        if (!sd[s].run_n) return;
-        const uint32_t* hw = h_out[s] ? fullh[s] : ctx->h_hist.as<uint32_t>() + s * (size_t)wn;
-        const int hn = h_out[s] ? R2 : wn, hb = h_out[s] ? 0 : wlo;
-        auto code_count = [&](uint32_t c) -> uint64_t {
-            return c >= (uint32_t)hb && c < (uint32_t)(hb + hn) ? hw[c - hb] : 0;
-        };
-        // runs only where they shorten the Huffman payload (else the decoder
-        // keeps its plain path): sum(count * length) of both codebooks
-        uint64_t bits_plain = 0;
-        for (size_t i = 0; i < syms[s].size(); ++i) bits_plain += code_count(syms[s][i]) * lens[s][i];
-        std::vector<std::pair<uint32_t, uint64_t>> set;
-        set.push_back({(uint32_t)o.radius, rstats[s * kRunStats]});
-        for (uint32_t i = 0; i < sd[s].run_n; ++i) set.push_back({sd[s].run_base + i, rstats[s * kRunStats + 1 + i]});
-        std::vector<uint16_t> rs;
-        std::vector<uint8_t> rl;
-        build_codebook_adjusted(hw, hn, hb, set, rs, rl);
-        uint64_t bits_runs = 0;
-        for (size_t i = 0; i < rs.size(); ++i) {
-            uint64_t c = code_count(rs[i]);
-            for (const auto& e : set)
-                if (e.first == rs[i]) c = e.second;
-            bits_runs += c * rl[i];
-        }
-        if (bits_runs < bits_plain) {
-            syms[s].swap(rs);
-            lens[s].swap(rl);
-        } else {
-            sd[s].run_n = 0;
-            sd[s].run_base = 0;
-        }
-    });
-    lap.mark("run codebooks");
-    uint32_t cb_total = 0;
-    for (int s = 0; s < nstreams; ++s) {
-        sd[s].cb_off = cb_total;
-        sd[s].n_used = (uint32_t)syms[s].size();
-        cb_total += sd[s].n_used;
-    }
-    // unpredictable values: per chunk list offsets
+    // unpredictable values: per chunk list offsets, gathered beside the coder
     std::vector<UnpredWork> uwork;
     std::vector<uint64_t> unpred_off(nstreams + 1, 0);
     for (int s = 0; s < nstreams; ++s) {
@@ -693,160 +689,53 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         unpred_off[s + 1] = acc;
     }
     const uint64_t total_unpred = unpred_off[nstreams];
-
-    // upload: sd | cb_sym | cb_len | work | ids | uwork
-    const size_t o_sd = 0, o_sym = align256(o_sd + sd.size() * sizeof(StreamDesc));
-    const size_t o_len = align256(o_sym + (size_t)cb_total * 2), o_work = align256(o_len + cb_total);
-    const size_t o_ids = align256(o_work + work.size() * sizeof(CtaWork));
-    const size_t o_uw = align256(o_ids + ids.size() * 4), up_bytes = align256(o_uw + uwork.size() * sizeof(UnpredWork));
-    STZ_CUDA(ctx->h_stage.ensure(up_bytes));
-    uint8_t* hs = ctx->h_stage.as<uint8_t>();
-    std::memcpy(hs + o_sd, sd.data(), sd.size() * sizeof(StreamDesc));
-    for (int s = 0; s < nstreams; ++s) {
-        std::memcpy(hs + o_sym + 2 * (size_t)sd[s].cb_off, syms[s].data(), 2 * syms[s].size());
-        std::memcpy(hs + o_len + sd[s].cb_off, lens[s].data(), lens[s].size());
-    }
-    std::memcpy(hs + o_work, work.data(), work.size() * sizeof(CtaWork));
-    std::memcpy(hs + o_ids, ids.data(), ids.size() * 4);
-    if (!uwork.empty()) std::memcpy(hs + o_uw, uwork.data(), uwork.size() * sizeof(UnpredWork));
-    STZ_CUDA(ctx->sd.ensure(up_bytes));
-    STZ_CUDA(cudaMemcpyAsync(ctx->sd.p, hs, up_bytes, cudaMemcpyHostToDevice, st));
-    uint8_t* dstage = ctx->sd.as<uint8_t>();
-    const StreamDesc* d_sd = (const StreamDesc*)(dstage + o_sd);
-    const uint16_t* d_sym = (const uint16_t*)(dstage + o_sym);
-    const uint8_t* d_len = (const uint8_t*)(dstage + o_len);
-    const CtaWork* d_work = (const CtaWork*)(dstage + o_work);
-    const uint32_t* d_ids = (const uint32_t*)(dstage + o_ids);
-    const UnpredWork* d_uw = (const UnpredWork*)(dstage + o_uw);
-
-    lap.mark("codebooks + upload");
-    // entropy coding
-    STZ_CUDA(ctx->ctab.ensure((size_t)nstreams * R2 * 4));
-    STZ_CUDA(ctx->sub_bits.ensure(g.total_sub * 4));
-    STZ_CUDA(ctx->sub_off.ensure(g.total_sub * 4));
-    STZ_CUDA(ctx->chunk_off.ensure(g.total_chunk_slots * 8));
-    STZ_CUDA(ctx->stream_words.ensure((size_t)nstreams * 8 * 3));
-    STZ_CUDA(ctx->payload.ensure(g.total_words * 4));
-    STZ_CUDA(ctx->ulist.ensure(std::max<uint64_t>(total_unpred, 1) * elem));
-    {
-        KScope ks(ctx, "k_expand_codebook");
-        launch_expand_codebook(d_sd, nstreams, d_sym, d_len, ctx->ctab.as<uint32_t>(), st);
-    }
-    STZ_CUDA(ctx->rbits.ensure((size_t)nstreams * kRunBitsStride));
-    {
-        KScope ks(ctx, "k_run_bits");
-        launch_run_bits(d_sd, nstreams, ctx->ctab.as<uint32_t>(), ctx->rbits.as<uint8_t>(), st);
-    }
-    {
-        KScope ks(ctx, "k_sub_bits");
-        launch_sub_bits(d_work, d_ids, (int)work.size(), d_sd, ctx->codes.as<uint16_t>(), ctx->ctab.as<uint32_t>(),
-                        ctx->rbits.as<uint8_t>(), ctx->sub_bits.as<uint32_t>(), st);
-    }
-    {
-        KScope ks(ctx, "k_scan_stream");
-        uint32_t max_chunks = 0;
-        for (int s = 0; s < nstreams; ++s) max_chunks = std::max(max_chunks, sd[s].nchunks);
-        launch_scan_streams(d_sd, nstreams, max_chunks, ctx->sub_bits.as<uint32_t>(), ctx->sub_off.as<uint32_t>(),
-                            ctx->chunk_off.as<uint64_t>(), ctx->stream_words.as<uint64_t>(),
-                            ctx->payload.as<uint32_t>(), st);
-    }
-    if (!uwork.empty()) {
-        KScope ks(ctx, "k_unpred_move");
-        launch_unpred_move<T>(true, d_uw, (int)uwork.size(), d_sd, ctx->codes.as<uint16_t>(),
-                              ctx->unpred_dense.as<T>(), ctx->ulist.as<T>(), st);
-    }
-    STZ_CUDA(cudaGetLastError());
-
-    // stream sizes and tables to the host (the payload is encoded next)
     const size_t t_words = 0, t_choff = align256(t_words + (size_t)nstreams * 8);
     const size_t t_sub = align256(t_choff + g.total_chunk_slots * 8);
     const size_t t_ul = align256(t_sub + g.total_sub * 4), t_bytes = align256(t_ul + total_unpred * elem);
     STZ_CUDA(ctx->h_io.ensure(t_bytes));
     uint8_t* ht = ctx->h_io.as<uint8_t>();
-    // on the copy stream, so the encode launches below do not wait for them
-    {
-        cudaEvent_t ev_scan = ctx->event();
-        STZ_CUDA(cudaEventRecord(ev_scan, st));
-        STZ_CUDA(cudaStreamWaitEvent(sc, ev_scan, 0));
-        ctx->ev_pool.push_back(ev_scan);  // the wait is enqueued: the event may be recorded again
+    if (!uwork.empty()) {
+        cudaStream_t su = ctx->st_side;
+        STZ_CUDA(ctx->ulist.ensure(total_unpred * elem));
+        STZ_CUDA(ctx->h_meta2.ensure(uwork.size() * sizeof(UnpredWork)));
+        std::memcpy(ctx->h_meta2.p, uwork.data(), uwork.size() * sizeof(UnpredWork));
+        STZ_CUDA(ctx->uwork.ensure(uwork.size() * sizeof(UnpredWork)));
+        STZ_CUDA(cudaStreamWaitEvent(su, named[EvUp], 0));
+        STZ_CUDA(cudaStreamWaitEvent(su, named[EvLevels], 0));
+        STZ_CUDA(cudaMemcpyAsync(ctx->uwork.p, ctx->h_meta2.p, uwork.size() * sizeof(UnpredWork),
+                                 cudaMemcpyHostToDevice, su));
+        {
+            KScope ks(ctx, "k_unpred_move", 1, su);
+            launch_unpred_move<T>(true, ctx->uwork.as<UnpredWork>(), (int)uwork.size(), d_sd,
+                                  ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(), ctx->ulist.as<T>(), su);
+        }
+        STZ_CUDA(cudaGetLastError());
+        STZ_CUDA(cudaMemcpyAsync(ht + t_ul, ctx->ulist.p, total_unpred * elem, cudaMemcpyDeviceToHost, su));
+        STZ_CUDA(cudaEventRecord(named[EvUnpred], su));
     }
+    lap.mark("unpredictable lists");
+
+    // codebooks, then the tables, on the copy stream
+    STZ_CUDA(cudaEventSynchronize(named[EvInfo]));
+    const CodebookInfo* cbi = (const CodebookInfo*)hb;
+    const uint64_t cb_total = (uint64_t)cbi[nstreams - 1].cb_off + cbi[nstreams - 1].n_used;
+    if (cb_total > cb_cap) STZ_FAIL(STZ_ERR_CUDA, "codebook kernel: more symbols than codes");
+    STZ_CUDA(cudaMemcpyAsync(hb + o_sym, d_sym, cb_total * 2, cudaMemcpyDeviceToHost, sc));
+    STZ_CUDA(cudaMemcpyAsync(hb + o_len, d_len, cb_total, cudaMemcpyDeviceToHost, sc));
+    const uint16_t* h_sym = (const uint16_t*)(hb + o_sym);
+    const uint8_t* h_len = hb + o_len;
+    for (int s = 0; s < nstreams; ++s) {
+        sd[s].cb_off = cbi[s].cb_off, sd[s].n_used = cbi[s].n_used;
+        sd[s].run_base = cbi[s].run_base, sd[s].run_n = cbi[s].run_n;
+    }
+    lap.mark("codebooks");
+    STZ_CUDA(cudaStreamWaitEvent(sc, named[EvScan], 0));
     STZ_CUDA(cudaMemcpyAsync(ht + t_words, ctx->stream_words.p, (size_t)nstreams * 8, cudaMemcpyDeviceToHost, sc));
     STZ_CUDA(cudaMemcpyAsync(ht + t_choff, ctx->chunk_off.p, g.total_chunk_slots * 8, cudaMemcpyDeviceToHost, sc));
     STZ_CUDA(cudaMemcpyAsync(ht + t_sub, ctx->sub_off.p, g.total_sub * 4, cudaMemcpyDeviceToHost, sc));
-    if (total_unpred)
-        STZ_CUDA(cudaMemcpyAsync(ht + t_ul, ctx->ulist.p, total_unpred * elem, cudaMemcpyDeviceToHost, sc));
-    struct Events {
-        std::vector<cudaEvent_t> e;
-        ~Events()
-        {
-            for (cudaEvent_t x : e) cudaEventDestroy(x);
-        }
-    } ev;
-    // Encode, pack and copy back in groups: every stream of the coarser
-    // levels, then the finest level's streams in two halves of their chunk
-    // z-layers (all 7 streams per group, so every launch still fills the
-    // device); the host zstd-compresses a group's frames while the device
-    // encodes the next (one, two, four or eight finest groups measured within
-    // noise of each other once payload frames skip zstd; two is the fewest
-    // launches that still overlap the copy back). The encodes are enqueued
-    // before the host waits for the tables; the copies once it has them.
-    const int fin0 = std::max(0, nstreams - 7);
-    const int fin_layers = (int)sd[nstreams - 1].ncz;
-    const int lpg = std::max(1, (fin_layers + 1) / 2);  // layers per group: two finest groups
-    const size_t ngroups = 1 + (size_t)((fin_layers + lpg - 1) / lpg);
-    // ev.e[gi]: group gi's words are on the host; ev.e[ngroups + gi]: its
-    // encode is done; ev.e[2 * ngroups]: the tables are on the host. The
-    // copies run on the context's copy stream, so group gi's copy overlaps
-    // group gi + 1's encode.
-    ev.e.assign(2 * ngroups + 1, nullptr);
-    // the pool's threads wait on the copy events ev.e[0, ngroups) while others
-    // compress frames: those waits block instead of spinning on a core
-    for (size_t i = 0; i < ev.e.size(); ++i)
-        STZ_CUDA(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming | (i < ngroups ? cudaEventBlockingSync : 0)));
-    STZ_CUDA(cudaEventRecord(ev.e[2 * ngroups], sc));
-    std::vector<CtaWork> gwork;
-    std::vector<uint32_t> gids;
-    std::vector<size_t> gw(ngroups + 1, 0);
-    for (int s = 0; s < fin0; ++s) add_all_chunks(gwork, gids, (uint32_t)s, sd[s].nchunks, (int)sd[s].C);
-    for (size_t gi = 1; gi < ngroups; ++gi) {
-        gw[gi] = gwork.size();
-        const int L0 = (int)(gi - 1) * lpg, L1 = std::min(fin_layers, L0 + lpg);
-        for (int s = fin0; s < nstreams; ++s) {
-            const uint32_t cpl = sd[s].ncx * sd[s].ncy;
-            std::vector<uint32_t> cs;
-            for (uint32_t c = (uint32_t)L0 * cpl; c < (uint32_t)L1 * cpl; ++c) cs.push_back(c);
-            add_work(gwork, gids, (uint32_t)s, cs.data(), cs.size(), (int)sd[s].C);
-        }
-    }
-    gw[0] = 0;
-    gw[ngroups] = gwork.size();
-    const size_t g_work = 0, g_ids = align256(gwork.size() * sizeof(CtaWork)), g_bytes = align256(g_ids + gids.size() * 4);
-    STZ_CUDA(ctx->h_meta2.ensure(g_bytes));
-    std::memcpy(ctx->h_meta2.as<uint8_t>() + g_work, gwork.data(), gwork.size() * sizeof(CtaWork));
-    std::memcpy(ctx->h_meta2.as<uint8_t>() + g_ids, gids.data(), gids.size() * 4);
-    STZ_CUDA(ctx->gwork.ensure(g_bytes));
-    STZ_CUDA(cudaMemcpyAsync(ctx->gwork.p, ctx->h_meta2.p, g_bytes, cudaMemcpyHostToDevice, st));
-    const CtaWork* d_gwork = (const CtaWork*)(ctx->gwork.as<uint8_t>() + g_work);
-    const uint32_t* d_gids = (const uint32_t*)(ctx->gwork.as<uint8_t>() + g_ids);
-    // the coarser levels' streams (group 0) are many small ones: packed back
-    // to back on the device, they go to the host in one transfer
-    if (fin0 > 0) STZ_CUDA(ctx->packed.ensure(sd[fin0].word_base * 4));
-    for (size_t gi = 0; gi < ngroups; ++gi) {
-        {
-            KScope ks(ctx, "k_encode");
-            launch_encode(d_gwork + gw[gi], d_gids, (int)(gw[gi + 1] - gw[gi]), d_sd, ctx->codes.as<uint16_t>(),
-                          ctx->ctab.as<uint32_t>(), ctx->rbits.as<uint8_t>(), ctx->sub_bits.as<uint32_t>(),
-                          ctx->sub_off.as<uint32_t>(), ctx->chunk_off.as<uint64_t>(), ctx->payload.as<uint32_t>(), st);
-        }
-        if (gi == 0 && fin0 > 0) {
-            KScope ks(ctx, "k_pack_streams");
-            launch_pack_streams(d_sd, ctx->stream_words.as<uint64_t>(), 0, fin0, ctx->payload.as<uint32_t>(),
-                                ctx->packed.as<uint32_t>(), st);
-        }
-        STZ_CUDA(cudaEventRecord(ev.e[ngroups + gi], st));
-    }
-    STZ_CUDA(cudaGetLastError());
-    STZ_CUDA(cudaEventSynchronize(ev.e[2 * ngroups]));
+    if (!uwork.empty()) STZ_CUDA(cudaStreamWaitEvent(sc, named[EvUnpred], 0));
+    STZ_CUDA(cudaEventRecord(named[EvTables], sc));
+    STZ_CUDA(cudaEventSynchronize(named[EvTables]));
     lap.mark("code lengths + tables");
     const uint64_t* words = (const uint64_t*)(ht + t_words);
 
@@ -928,7 +817,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     // finest streams', the largest, first)
     auto build_header = [&](size_t s) {
         const StreamDesc& d = sd[s];
-        append_stream_header(parts[s].hdr, syms[s].data(), lens[s].data(), d.n_used, d.run_base, d.run_n,
+        append_stream_header(parts[s].hdr, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
                              unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
                              h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
                              (int)d.C);
@@ -960,6 +849,9 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         STZ_CUDA(cudaStreamSynchronize(st));
     }
     STZ_CUDA(cudaStreamSynchronize(ctx->st_copy));  // every group's copy (the payload buffer is reused next call)
+    if (level_error_take()) STZ_FAIL(STZ_ERR_CUDA, "level kernel: a TMA tile load did not complete in time");
+    if (M && M->mask && learned_tc_error_take(st))
+        STZ_FAIL(STZ_ERR_CUDA, "learned correction: a tensor-core MMA did not complete in time");
     lap.mark("encode + copy + zstd");
     auto* so = new (std::nothrow) stz_stream();
     if (!so) STZ_FAIL(STZ_ERR_NOMEM, "out of host memory");
@@ -2288,7 +2180,7 @@ stz_status stz_debug_codebook(const uint32_t* hist, int nbins, uint16_t* sym, ui
     if (!hist || !sym || !len || !n_used || nbins <= 0 || nbins > 65536) STZ_FAIL(STZ_ERR_ARG, "bad arguments");
     std::vector<uint16_t> s;
     std::vector<uint8_t> l;
-    const int n = build_codebook(hist, nbins, 0, s, l);
+    const int n = build_codebook(hist, nbins, s, l);
     std::memcpy(sym, s.data(), 2 * (size_t)n);
     std::memcpy(len, l.data(), (size_t)n);
     *n_used = n;

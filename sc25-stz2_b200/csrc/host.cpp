@@ -169,14 +169,7 @@ void min_redundancy_lengths(std::vector<uint64_t>& a)
 
 }  // namespace
 
-int build_codebook(const uint32_t* hist, int nbins, int base, std::vector<uint16_t>& sym, std::vector<uint8_t>& len)
-{
-    return build_codebook_adjusted(hist, nbins, base, {}, sym, len);
-}
-
-int build_codebook_adjusted(const uint32_t* hist, int nbins, int base,
-                            const std::vector<std::pair<uint32_t, uint64_t>>& set, std::vector<uint16_t>& sym,
-                            std::vector<uint8_t>& len)
+int build_codebook(const uint32_t* hist, int nbins, std::vector<uint16_t>& sym, std::vector<uint8_t>& len)
 {
     struct Item {
         uint64_t w;
@@ -184,16 +177,7 @@ int build_codebook_adjusted(const uint32_t* hist, int nbins, int base,
     };
     std::vector<Item> items;
     for (int i = 0; i < nbins; ++i)
-        if (hist[i]) items.push_back({hist[i], (uint32_t)(i + base)});
-    if (!set.empty()) {  // items are in symbol order: replace or append the set's counts
-        for (const auto& o : set) {
-            auto it = std::lower_bound(items.begin(), items.end(), o.first,
-                                       [](const Item& x, uint32_t sym) { return x.s < sym; });
-            if (it != items.end() && it->s == o.first) it->w = o.second;
-            else items.insert(it, {o.second, o.first});
-        }
-        items.erase(std::remove_if(items.begin(), items.end(), [](const Item& x) { return x.w == 0; }), items.end());
-    }
+        if (hist[i]) items.push_back({hist[i], (uint32_t)i});
     const int n = (int)items.size();
     sym.clear();
     len.clear();

@@ -82,13 +82,9 @@ private:
 // algorithm of Moffat & Katajainen); lengths capped at kMaxCodeLen by
 // lengthening the least frequent code below the cap until the Kraft sum fits;
 // output in canonical (length, symbol) order. A lone symbol gets length 0.
-// `base` is added to every histogram index (windowed histograms).
-int build_codebook(const uint32_t* hist, int nbins, int base, std::vector<uint16_t>& sym, std::vector<uint8_t>& len);
-// The same with the counts of the listed symbols set (symbols outside the
-// window [base, base + nbins) are added).
-int build_codebook_adjusted(const uint32_t* hist, int nbins, int base,
-                            const std::vector<std::pair<uint32_t, uint64_t>>& set, std::vector<uint16_t>& sym,
-                            std::vector<uint8_t>& len);
+// The host's statement of the rule (compress builds its codebooks on the
+// device, codebook.cu).
+int build_codebook(const uint32_t* hist, int nbins, std::vector<uint16_t>& sym, std::vector<uint8_t>& len);
 
 // ---- run symbols (container version 3) ---------------------------------------
 // Runs of the centre code (= radius) inside a plane are coded with run

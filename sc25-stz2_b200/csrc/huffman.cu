@@ -31,42 +31,10 @@
 #include <cuda_runtime.h>
 
 #include "huffman.h"
+#include "run_symbols.cuh"
 
 namespace stz {
 namespace {
-
-// Canonical codes from the (length, symbol)-sorted list: first code of each
-// length by the usual recurrence, then rank within the length.
-__global__ void k_expand_codebook(const StreamDesc* __restrict__ sd, const uint16_t* __restrict__ cb_sym,
-                                  const uint8_t* __restrict__ cb_len, uint32_t* __restrict__ ctab)
-{
-    const StreamDesc s = sd[blockIdx.x];
-    __shared__ uint32_t cnt[kMaxCodeLen + 1];
-    __shared__ uint32_t first_code[kMaxCodeLen + 1];
-    __shared__ uint32_t first_idx[kMaxCodeLen + 1];
-    if (threadIdx.x <= kMaxCodeLen) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < s.n_used; i += blockDim.x) atomicAdd(&cnt[cb_len[s.cb_off + i]], 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t code = 0, idx = cnt[0];
-        first_code[0] = 0;
-        first_idx[0] = 0;
-        for (int l = 1; l <= kMaxCodeLen; ++l) {
-            code = (code + (l > 1 ? cnt[l - 1] : 0)) << 1;
-            first_code[l] = code;
-            first_idx[l] = idx;
-            idx += cnt[l];
-        }
-    }
-    __syncthreads();
-    uint32_t* tab = ctab + (size_t)blockIdx.x * 2 * s.radius;
-    for (uint32_t i = threadIdx.x; i < s.n_used; i += blockDim.x) {
-        const uint32_t l = cb_len[s.cb_off + i];
-        const uint32_t code = l ? first_code[l] + (i - first_idx[l]) : 0;
-        tab[cb_sym[s.cb_off + i]] = (code << 5) | l;
-    }
-}
 
 // ---- encode side: a lane group per plane ----------------------------------------
 // (Planes of up to 1024 codes take the literal lists below; this segment form
@@ -83,27 +51,6 @@ __global__ void k_expand_codebook(const StreamDesc* __restrict__ sd, const uint1
 // bitstream is the one a sequential pass over the plane writes.
 constexpr int kLaneThreads = 256;  // 8 warps per CTA, each one plane at a time
 constexpr int kPlaneSlices = 4;    // CTAs per work item (gridDim.y)
-
-// Symbols of a run of r centre codes (none for r = 0), in order: while
-// r > D, 2^k (the largest power of two <= r, k <= J) when k > LD, else D
-// codes; then the symbol of the remaining 2..D codes, or the centre code.
-template <class F>
-__device__ __forceinline__ void run_symbols(uint32_t r, uint32_t R, uint32_t base, uint32_t J, uint32_t D, uint32_t LD,
-                                            F&& f)
-{
-    while (r > D) {
-        const uint32_t k = min((uint32_t)(31 - __clz(r)), J);
-        if (k > LD) {
-            f(base + D - 1 + (k - LD - 1));
-            r -= 1u << k;
-        } else {
-            f(base + D - 2);
-            r -= D;
-        }
-    }
-    if (r >= 2) f(base + r - 2);
-    else if (r) f(R);
-}
 
 // Lanes per plane: the largest power of two <= plane / 32, at most 32, so a
 // lane holds about 32 codes; a warp takes 32 / W planes at a time (small
@@ -352,24 +299,6 @@ __device__ __forceinline__ void literal_rounds2(const uint16_t* list, uint32_t L
 __device__ __forceinline__ uint32_t tail_run(const uint16_t* list, uint32_t L, uint32_t P)
 {
     return P - (L ? list[L - 1] + 1u : 0u);
-}
-
-// Bits of the run symbols of a run of r centre codes (r <= P), per stream:
-// rb[r], r = 0 .. kRunBitsStride - 1 (planes of up to 1024 codes).
-__global__ void k_run_bits(const StreamDesc* __restrict__ sd, const uint32_t* __restrict__ ctab,
-                           uint8_t* __restrict__ rbits)
-{
-    const StreamDesc s = sd[blockIdx.x];
-    const uint32_t P = s.C * s.C;
-    if (s.run_n == 0 || P >= kRunBitsStride) return;
-    const uint32_t* tab = ctab + (size_t)blockIdx.x * 2 * s.radius;
-    uint32_t D, LD;
-    const uint32_t J = run_geometry(P, D, LD);
-    for (uint32_t r = threadIdx.x; r <= P; r += blockDim.x) {
-        uint32_t b = 0;
-        run_symbols(r, s.radius, s.run_base, J, D, LD, [&](uint32_t sym) { b += __ldg(tab + sym) & 31u; });
-        rbits[(size_t)blockIdx.x * kRunBitsStride + r] = (uint8_t)b;
-    }
 }
 
 // Run-symbol counts of every listed plane (streams with runs).
@@ -1342,21 +1271,10 @@ void launch_pack_streams(const StreamDesc* sd, const uint64_t* stream_words, int
     if (s1 > s0) k_pack_streams<<<dim3(16, s1 - s0), 256, 0, st>>>(sd, stream_words, s0, payload, dst);
 }
 
-void launch_expand_codebook(const StreamDesc* sd, int nstreams, const uint16_t* cb_sym, const uint8_t* cb_len,
-                            uint32_t* ctab, cudaStream_t st)
-{
-    if (nstreams) k_expand_codebook<<<nstreams, 256, 0, st>>>(sd, cb_sym, cb_len, ctab);
-}
-
 void launch_run_stats(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
                       const uint16_t* codes, unsigned long long* stats, cudaStream_t st)
 {
     if (nwork > 0) k_run_stats<<<dim3(nwork, kPlaneSlices), kLaneThreads, 0, st>>>(work, chunk_ids, sd, codes, stats);
-}
-
-void launch_run_bits(const StreamDesc* sd, int nstreams, const uint32_t* ctab, uint8_t* rbits, cudaStream_t st)
-{
-    if (nstreams) k_run_bits<<<nstreams, 256, 0, st>>>(sd, ctab, rbits);
 }
 
 void launch_sub_bits(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,

@@ -17,22 +17,33 @@ struct UnpredWork {
     uint64_t count;  // values of this chunk in the list
 };
 
-// Dense code table per stream (2*radius entries): code << 5 | length.
-void launch_expand_codebook(const StreamDesc* sd, int nstreams, const uint16_t* cb_sym, const uint8_t* cb_len,
-                            uint32_t* ctab, cudaStream_t st);
 // Run-symbol counts per stream (streams with run_n > 0): stats[s * kRunStats]
 // gets the centre codes left as single symbols, stats[s * kRunStats + 1 + i]
 // the uses of run slot i. stats must be zeroed.
 constexpr int kRunStats = 64;
 // Per stream: the bits of a run of r centre codes, r < kRunBitsStride
-// (launch_run_bits; planes of up to 1024 codes).
+// (launch_codebooks; planes of up to 1024 codes).
 constexpr uint32_t kRunBitsStride = 1025;
 void launch_run_stats(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
                       const uint16_t* codes, unsigned long long* stats, cudaStream_t st);
-// Bits of a run of r centre codes per stream (rbits: nstreams x
-// kRunBitsStride bytes), from the stream's code table (after
-// launch_expand_codebook); streams with runs and planes of up to 1024 codes.
-void launch_run_bits(const StreamDesc* sd, int nstreams, const uint32_t* ctab, uint8_t* rbits, cudaStream_t st);
+// Codebooks of every stream from its code histogram (2 radius bins a stream),
+// the counts of codes outside the host window's range and the run-symbol
+// counts (codebook.cu): patches each descriptor's cb_off, n_used, run_base
+// and run_n, and writes the code tables (ctab: 2 radius entries a stream, code
+// << 5 | length), the bits of a run of r centre codes (rbits: nstreams x
+// kRunBitsStride bytes; streams with runs and planes of up to 1024 codes),
+// the canonical (symbol, length) lists of all streams back to back, and what
+// the host needs to find them. scratch_off[q]: first scratch item of stream
+// q, codebook_items(stream) items each; items: their total.
+struct CodebookInfo {
+    uint32_t cb_off, n_used, run_base, run_n;
+};
+uint64_t codebook_items(const StreamDesc& s, uint64_t codes);
+size_t codebook_scratch_bytes(uint64_t items, int nstreams);
+void launch_codebooks(StreamDesc* sd, int nstreams, const uint32_t* hist, const uint32_t* outside,
+                      const unsigned long long* rstats, const uint64_t* scratch_off, uint64_t items, void* scratch,
+                      uint32_t* ctab, uint8_t* rbits, uint16_t* cb_sym, uint8_t* cb_len, CodebookInfo* info,
+                      cudaStream_t st);
 void launch_sub_bits(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
                      const uint16_t* codes, const uint32_t* ctab, const uint8_t* rbits, uint32_t* sub_bits,
                      cudaStream_t st);
