@@ -11,11 +11,9 @@
 // Parallel decomposition: every z-plane of a chunk (C^2 symbols, a
 // "sub-chunk") has its bit offset inside the chunk in the stream header, so
 // all planes of all chunks of all streams encode and decode independently.
-// Inside a plane, a group of lanes shares the work: the encode side splits
-// the codes into lane segments (runs are the gaps between literal masks),
-// the decoder splits the bits into lane slices and resynchronises them
-// (a dense stream in a large launch is decoded one thread per plane
-// instead). Bits are packed MSB-first into 32-bit words; a chunk starts on a
+// Inside a plane, the encode side shares the codes among a group of lanes
+// (runs are the gaps between literal masks); the decoder gives a lane to each
+// plane. Bits are packed MSB-first into 32-bit words; a chunk starts on a
 // word boundary.
 //
 // Runs: inside a plane, a maximal run of r centre codes (code == radius) is
@@ -26,8 +24,6 @@
 // so they share the codebook, the tables and the 16-bit symbol width with
 // the codes; a well-predicted stream (mostly centre codes) then costs well
 // under one bit per code.
-#include <cstdlib>
-
 #include <cuda_runtime.h>
 
 #include "huffman.h"
@@ -664,443 +660,453 @@ __global__ void __launch_bounds__(kLaneThreads) k_encode(const CtaWork* __restri
     }
 }
 
-// Decode: a warp decodes one plane with a 2^kLutBits-entry table in shared
-// memory (symbol | length << 16); longer codes fall back to the canonical
-// first-code test per length.
-// Symbols of codes longer than kLutBits kept with the tables (the rest of a
-// longer tail is read from the codebook).
-constexpr int kTailSyms = 4096;
+// ---- decode: a lane group per plane ----------------------------------------------
+// Parallel Huffman decoding by self-synchronisation (Weissenberger & Schmidt,
+// "Massively parallel Huffman decoding on GPUs", ICPP 2018): a plane's bits
+// are cut into W slices; lane i decodes the codes that start in its slice,
+// beginning at the slice start. A lane whose start is not where its left
+// neighbour's last code ends decodes again from there, until no start moves
+// (codes resynchronise within 5 to 20 symbols, so one to five rounds are
+// usual). A scan of the lanes' code counts (a run symbol counts its run) then
+// places each lane's literals.
+// A symbol is decoded about three times, so the kernel is bound by the
+// instructions and the latency of that step, and everything it reads lies in
+// shared memory: the stream's table, the plane's payload words (copied there
+// first, asynchronously), and the plane's codes, which start out as centre
+// codes, take the literals, and are stored at the end, 16 bytes a lane.
+//   * One lookup gives the length of any code but the few whose table prefix
+//     spans two lengths: canonical codes of one length are one interval. A
+//     code of up to kLutBits bits also gets its symbol or run length, a
+//     longer one its canonical index.
+//   * The symbols of longer codes are looked up when the plane is stored,
+//     many at a time, so no lane waits for one in the middle of its chain.
+//     Where long codes are common (DecodeTables::by_index) the plane holds
+//     indexes only.
+// Before, table, payload words and symbols were read through L1 in the chain,
+// the length of a long code was searched there, and dense streams of large
+// launches had one thread per plane, whose lanes diverged. Launch times on one
+// B200, before and now (levels below the finest, then its two halves):
+//   512^3 f32 at 1e-3          0.139 / 0.160 / 0.131 -> 0.127 / 0.166 / 0.126 ms
+//   512^3 f32 at 1e-4          0.221 / 1.036 / 0.711 -> 0.198 / 0.496 / 0.315 ms
+//   384x384x256 f64 at 1e-6    0.230 / 0.560 / 0.520 -> 0.079 / 0.270 / 0.229 ms
+//   its boxes of 16-128 a side 0.156 -> 0.068 ms a box
+// Tried as well: one lane per plane in lockstep (windows of codes in shared
+// memory, payload rings filled by asynchronous copies), 0.17 / 0.62 / 0.42 ms
+// at 1e-4 and a chain of 1024 symbols in every small launch; several symbols
+// per lookup in the counting passes (fewer instructions, more table to load:
+// even); four lanes' worth of planes per warp for all streams (fewer warps
+// resident: slower).
 
-// Decode tables of one stream, built once per prepared stream in device
-// memory (k_build_tables) and read by the decoders through L1.
-// lut entry: sym | len << 16 for codes of at most kLutBits bits; for a prefix
-// of longer codes, l_min << 24 with l_min the shortest code length under that
-// prefix (the canonical length search starts there); 0 for a prefix of no code.
+// lut entry: code length in bits 0-4 (0: the prefix spans lengths, holds long
+// run symbols, or no code); kLutRun: a run symbol, its run length in
+// bits 16-31; kLutLong: a longer code, its canonical index is its value plus
+// bits 16-31 (mod 2^16); else the symbol in bits 16-31 (its canonical index
+// where the stream decodes by index).
+constexpr uint32_t kLutRun = 0x100u, kLutLong = 0x200u;
 struct DecodeTables {
     uint32_t lut[1 << kLutBits];
-    uint32_t cnt[kMaxCodeLen + 1];
-    uint32_t first_code[kMaxCodeLen + 1];
-    uint32_t first_idx[kMaxCodeLen + 1];
-    uint16_t tail[kTailSyms];
+    // per code length: limit (codes of up to that length lie below it, as
+    // left-aligned kMaxCodeLen-bit numbers), the canonical index of a code
+    // minus its value, the first index of its run symbols, and their count
+    // (bits 0-15) and place in run (bits 16-31)
+    uint4 len[kMaxCodeLen + 1];
+    uint16_t run[64];   // run lengths, in canonical order
+    uint32_t max_len;   // longest code
+    uint32_t by_index;  // decode canonical indexes, look symbols up at the store
 };
 
+constexpr int kBuildThreads = 512;
+
 // One CTA per stream.
-__global__ void __launch_bounds__(256) k_build_tables(const StreamDesc* __restrict__ sd,
-                                                      const uint16_t* __restrict__ cb_sym,
-                                                      const uint8_t* __restrict__ cb_len,
-                                                      DecodeTables* __restrict__ out)
+__global__ void __launch_bounds__(kBuildThreads) k_build_tables(const StreamDesc* __restrict__ sd,
+                                                                const uint16_t* __restrict__ cb_sym,
+                                                                const uint8_t* __restrict__ cb_len,
+                                                                DecodeTables* __restrict__ out)
 {
     const StreamDesc s = sd[blockIdx.x];
     DecodeTables& t = out[blockIdx.x];
-    __shared__ uint32_t cnt[kMaxCodeLen + 1];
-    __shared__ uint32_t first_code[kMaxCodeLen + 1];
-    __shared__ uint32_t first_idx[kMaxCodeLen + 1];
-    if (threadIdx.x <= kMaxCodeLen) cnt[threadIdx.x] = 0;
+    __shared__ uint32_t cnt[kMaxCodeLen + 1], first_code[kMaxCodeLen + 1], first_idx[kMaxCodeLen + 1];
+    __shared__ uint32_t start[kMaxCodeLen + 1];  // first index of each length (the list is in length order)
+    __shared__ uint32_t rlo[kMaxCodeLen + 1], rcnt[kMaxCodeLen + 1], roff[kMaxCodeLen + 1];
+    __shared__ uint32_t by_index;
+    const uint32_t tid = threadIdx.x;
+    if (tid <= kMaxCodeLen) start[tid] = 0xffffffffu, rlo[tid] = 0xffffffffu, rcnt[tid] = 0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < s.n_used; i += blockDim.x) atomicAdd(&cnt[cb_len[s.cb_off + i]], 1u);
+    uint32_t D, LD;
+    run_geometry(s.C * s.C, D, LD);
+    for (uint32_t i = tid; i < s.n_used; i += kBuildThreads) {
+        const uint32_t l = cb_len[s.cb_off + i];
+        if (i == 0 || cb_len[s.cb_off + i - 1] != l) start[l] = i;
+        if ((uint32_t)cb_sym[s.cb_off + i] - s.run_base < s.run_n) {
+            atomicMin(&rlo[l], i);
+            atomicAdd(&rcnt[l], 1u);
+        }
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t code = 0, idx = cnt[0];
-        first_code[0] = 0;
-        first_idx[0] = 0;
+    if (tid == 0) {
+        for (int l = kMaxCodeLen, end = (int)s.n_used; l >= 0; --l) {
+            cnt[l] = start[l] == 0xffffffffu ? 0u : (uint32_t)end - start[l];
+            if (cnt[l]) end = (int)start[l];
+        }
+        uint32_t code = 0, idx = cnt[0], ro = 0, longest = 0, mass = 0;
+        first_code[0] = first_idx[0] = roff[0] = 0;
         for (int l = 1; l <= kMaxCodeLen; ++l) {
             code = (code + (l > 1 ? cnt[l - 1] : 0)) << 1;
             first_code[l] = code;
             first_idx[l] = idx;
             idx += cnt[l];
+            roff[l] = ro;
+            ro += rcnt[l];
+            if (cnt[l]) longest = l;
+            if (l <= kLutBits) mass += cnt[l] << (kLutBits - l);
         }
+        t.max_len = longest;
+        // more than one symbol in 128 has a long code
+        by_index = t.by_index = (1u << kLutBits) - mass > (1u << kLutBits) / 128 && longest > kLutBits;
     }
     __syncthreads();
-    if (threadIdx.x <= kMaxCodeLen) {
-        t.cnt[threadIdx.x] = cnt[threadIdx.x];
-        t.first_code[threadIdx.x] = first_code[threadIdx.x];
-        t.first_idx[threadIdx.x] = first_idx[threadIdx.x];
-    }
-    // every table entry finds its code: the shortest length whose canonical
-    // range holds the entry's prefix; prefixes of longer codes record the
-    // shortest such length
-    for (uint32_t j = threadIdx.x; j < (1u << kLutBits); j += blockDim.x) {
-        uint32_t e = 0;
-        for (uint32_t l = 1; l <= (uint32_t)kLutBits; ++l) {
-            const uint32_t v = (j >> (kLutBits - l)) - first_code[l];
-            if (v < cnt[l]) {
-                e = (uint32_t)cb_sym[s.cb_off + first_idx[l] + v] | (l << 16);
-                break;
-            }
+    if (tid <= kMaxCodeLen)
+        t.len[tid] = make_uint4(tid ? (first_code[tid] + cnt[tid]) << (kMaxCodeLen - tid) : 0u,
+                                first_idx[tid] - first_code[tid], rlo[tid], rcnt[tid] | roff[tid] << 16);
+    // run lengths in canonical order: run symbols of one length are consecutive
+    for (uint32_t i = tid; i < s.n_used; i += kBuildThreads) {
+        const uint32_t r = (uint32_t)cb_sym[s.cb_off + i] - s.run_base;
+        if (r < s.run_n) {
+            const uint32_t l = cb_len[s.cb_off + i];
+            t.run[roff[l] + i - rlo[l]] = (uint16_t)run_length(r, D, LD);
         }
-        if (!e) {
-            for (uint32_t l = kLutBits + 1; l <= (uint32_t)kMaxCodeLen; ++l) {
-                if (!cnt[l]) continue;
-                const uint32_t sh = l - kLutBits;
-                if (j >= (first_code[l] >> sh) && j <= ((first_code[l] + cnt[l] - 1) >> sh)) {
-                    e = l << 24;
-                    break;
+    }
+    // the shortest length whose canonical range holds the entry's prefix, or
+    // the one longer length all codes under the prefix have
+    for (uint32_t j = tid; j < (1u << kLutBits); j += kBuildThreads) {
+        uint32_t e = 0;
+        for (uint32_t l = 1; l <= (uint32_t)kMaxCodeLen && !e; ++l) {
+            if (l <= (uint32_t)kLutBits) {
+                const uint32_t v = (j >> (kLutBits - l)) - first_code[l];
+                if (v < cnt[l]) {
+                    const uint32_t i = first_idx[l] + v, sym = cb_sym[s.cb_off + i], r = sym - s.run_base;
+                    e = l | (r < s.run_n ? kLutRun | run_length(r, D, LD) << 16 : (by_index ? i : sym) << 16);
                 }
+            } else {
+                const uint32_t sh = l - kLutBits, lo = j << sh, hi = lo + (1u << sh) - 1, b = first_idx[l] - first_code[l];
+                if (lo >= first_code[l] && hi < first_code[l] + cnt[l] &&
+                    (!rcnt[l] || hi + b < rlo[l] || lo + b >= rlo[l] + rcnt[l]))
+                    e = l | kLutLong | b << 16;
             }
         }
         t.lut[j] = e;
     }
-    const uint32_t t0 = first_idx[kLutBits + 1];
-    for (uint32_t i = threadIdx.x; i < (uint32_t)kTailSyms && t0 + i < s.n_used; i += blockDim.x)
-        t.tail[i] = cb_sym[s.cb_off + t0 + i];
 }
 
-// The symbol whose code starts at the top of `bits` (MSB first, at least
-// kMaxCodeLen valid bits); its code length in l (>= 1). A prefix of no code
-// (corrupt stream) yields the codebook's first symbol with length 1, so
-// every step consumes a bit.
-__device__ __forceinline__ uint32_t lookup_symbol(const DecodeTables* __restrict__ t, const StreamDesc& s,
-                                                  const uint16_t* __restrict__ cb_sym, uint32_t bits, uint32_t& l)
-{
-    const uint32_t e = __ldg(&t->lut[bits >> (32 - kLutBits)]);
-    uint32_t sym = e & 0xffffu;
-    l = (e >> 16) & 0xffu;
-    if (!l) {
-        // canonical search from the shortest length under this prefix
-        l = e >> 24;
-        if (!l) l = kLutBits + 1;
-        for (; l <= (uint32_t)kMaxCodeLen; ++l) {
-            const uint32_t v = bits >> (32 - l), fc = __ldg(&t->first_code[l]);
-            if (v - fc < __ldg(&t->cnt[l])) {
-                const uint32_t fi = __ldg(&t->first_idx[l]);
-                const uint32_t idx = fi + (v - fc);
-                const uint32_t ti = idx - __ldg(&t->first_idx[kLutBits + 1]);
-                sym = ti < (uint32_t)kTailSyms ? __ldg(&t->tail[ti]) : cb_sym[s.cb_off + idx];
-                break;
-            }
-        }
-        if (l > (uint32_t)kMaxCodeLen) {
-            sym = cb_sym[s.cb_off];
-            l = 1;
-        }
-    }
-    return sym;
-}
+constexpr int kDecodeWarps = 8;
+constexpr int kDecodeThreads = 32 * kDecodeWarps;
+constexpr uint32_t kMaxPlane = 1024;    // planes of up to this many codes fit the shared buffers
+constexpr uint32_t kStageWords = 512;   // payload words of the planes a warp decodes at a time
+constexpr uint32_t kNoIndex = 0xffffu;  // a plane's entry without a literal (by_index)
 
-// Bits of one chunk's payload: 32 bits from any bit position. Plane bit
-// ranges are validated against the chunk's words, and every stream keeps at
-// least two words of zero padding after its payload, so a read at a position
-// below a plane's end stays inside the stream's buffer.
-struct ChunkBits {
-    const uint32_t* in;
-    __device__ __forceinline__ uint32_t peek(uint32_t pos) const
+struct DecodeSmem {
+    uint32_t lut[1 << kLutBits];
+    uint4 out[kDecodeWarps][kMaxPlane / 8];
+    uint4 stage[kDecodeWarps][kStageWords / 4];
+    uint32_t late[kDecodeWarps][kMaxPlane / 32];  // entries that hold the index of a long code
+};
+
+// Symbol decoding from a stream's tables, the lookup table itself in shared
+// or in global memory.
+struct DecodeCtx {
+    const uint32_t* lut;
+    const DecodeTables* __restrict__ t;
+    // The code at the top of bits: its length, and symbol or run length, or
+    // canonical index (late).
+    template <bool SMEM>
+    __device__ __forceinline__ void symbol(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
     {
-        const uint32_t i = pos >> 5;
-        return __funnelshift_l(__ldg(in + i + 1), __ldg(in + i), pos & 31);
+        const uint32_t e = SMEM ? lut[bits >> (32 - kLutBits)] : __ldg(lut + (bits >> (32 - kLutBits)));
+        l = e & 31u, val = e >> 16, run = e & kLutRun, late = e & kLutLong;
+        if (late) val = (bits >> (32 - l)) + val & 0xffffu;
+        if (l == 0) slow(bits, l, val, run, late);
+    }
+    __device__ __forceinline__ void slow(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
+    {
+        const uint32_t v = bits >> (32 - kMaxCodeLen), longest = __ldg(&t->max_len);
+        l = kLutBits + 1;
+        while (l <= longest && v >= __ldg(&t->len[l].x)) ++l;
+        run = false, late = true;
+        if (l > longest) {  // no code (corrupt stream): the codebook's first symbol, one bit
+            l = 1;
+            val = 0;
+            return;
+        }
+        const uint4 e = __ldg(&t->len[l]);
+        const uint32_t i = (bits >> (32 - l)) + e.y, r = i - e.z;
+        run = r < (e.w & 0xffffu);
+        val = run ? __ldg(&t->run[(e.w >> 16) + r]) : i;
     }
 };
 
-// Decode every code that starts in [pos, stop): f(sym) for each; returns the
-// position after the last one (the first code boundary >= stop, or pos).
-template <class F>
-__device__ __forceinline__ uint32_t decode_range(const DecodeTables* __restrict__ t, const StreamDesc& s,
-                                                 const uint16_t* __restrict__ cb_sym, const ChunkBits& cb,
-                                                 uint32_t pos, uint32_t stop, F&& f)
+// 32 bits of a plane from any bit position; the words lie in shared or in
+// global memory, and at least two more follow every plane's in the same
+// buffer (a stream keeps four words after its payload).
+template <class Words>
+__device__ __forceinline__ uint32_t peek(const Words& w, uint32_t pos)
 {
-    while (pos < stop) {
-        uint32_t l;
-        const uint32_t sym = lookup_symbol(t, s, cb_sym, cb.peek(pos), l);
-        pos += l;
-        f(sym);
-    }
-    return pos;
+    return __funnelshift_l(w((pos >> 5) + 1), w(pos >> 5), pos);
 }
 
-// Decode plane lz of chunk c of stream s (one thread, sequentially): for
-// dense streams, where a plane holds many symbols and a warp per plane would
-// decode each one about three times.
-__device__ void decode_plane_seq(const DecodeTables* __restrict__ t, const StreamDesc& s, uint32_t c, uint32_t lz,
-                             const uint16_t* __restrict__ cb_sym, const uint32_t* __restrict__ sub_off,
-                             const uint64_t* __restrict__ chunk_word_off, const uint32_t* __restrict__ payload,
-                             uint16_t* __restrict__ codes)
+// Decode the plane of bits [r0, r1) by this lane's group of W lanes: the
+// literals go to put(code, value, late).
+template <bool SMEM, class Words, class Put>
+__device__ __forceinline__ void decode_plane(const DecodeCtx& dc, const Words& w, uint32_t r0, uint32_t r1, uint32_t W,
+                                             uint32_t lane, Put&& put)
 {
-    const uint32_t* __restrict__ lut = t->lut;
-    const uint32_t* __restrict__ cnt = t->cnt;
-    const uint32_t* __restrict__ first_code = t->first_code;
-    const uint32_t* __restrict__ first_idx = t->first_idx;
-    const uint32_t C = s.C;
-    const size_t plane = (size_t)C * C;
-    uint16_t* dst = codes + s.code_off + (size_t)c * plane * C + (size_t)lz * plane;
-    if (s.n_used == 1) {
-        // a lone run symbol means the plane is all centre codes
-        const uint16_t v0 = cb_sym[s.cb_off];
-        const uint16_t v = (uint32_t)v0 - s.run_base < s.run_n ? (uint16_t)s.radius : v0;
-        if (plane % 8 == 0 && ((uintptr_t)dst & 15) == 0) {
-            const uint32_t v2 = (uint32_t)v | ((uint32_t)v << 16);
-            for (size_t j = 0; j < plane / 8; ++j) reinterpret_cast<uint4*>(dst)[j] = make_uint4(v2, v2, v2, v2);
-        } else {
-            for (size_t j = 0; j < plane; ++j) dst[j] = v;
-        }
-        return;
-    }
-    const uint64_t cw = chunk_word_off[s.chunk_base + c];
-    const uint32_t* in = payload + s.word_base + cw;
-    // words of the stream left from this chunk's start; reads beyond read 0
-    const uint64_t lim = s.word_cap > cw ? s.word_cap - cw : 0;
-    auto rd = [&](uint64_t i) -> uint32_t { return i < lim ? __ldg(in + i) : 0u; };
-    uint32_t pos = sub_off[s.sub_base + (size_t)c * C + lz];  // bit position from the chunk's first word
-    // The plane's payload lines are prefetched into L1 up front (its end is
-    // the next plane's start, or the chunk's end), so the loads below hit L1.
-    {
-        const uint64_t cwords = chunk_word_off[s.chunk_base + c + 1] - cw;
-        const uint64_t b1 = lz + 1 < C ? (uint64_t)sub_off[s.sub_base + (size_t)c * C + lz + 1] : 32 * cwords;
-        const uint64_t w1 = min(min((b1 + 31) >> 5, cwords) + 2, lim);
-        for (uint64_t w = (pos >> 5) & ~31u; w < w1; w += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(in + w));
-    }
-    // 64-bit bit reservoir, MSB = next bit, `avail` valid bits (>= kLutBits
-    // at every symbol start). The dependency chain of a symbol is only
-    // table index -> lookup -> length -> shift: the refill word is merged in
-    // (below the valid bits, from the length-independent `avail`) while the
-    // lookup is in flight, and the next word is loaded one refill ahead.
-    uint64_t wi = pos >> 5;
-    uint64_t buf = (((uint64_t)rd(wi) << 32) | rd(wi + 1)) << (pos & 31);
-    int avail = 64 - (int)(pos & 31);
-    uint32_t w = rd(wi + 2);
-    wi += 3;
-    auto next = [&]() -> uint32_t {
-        const uint32_t e = __ldg(lut + (uint32_t)(buf >> (64 - kLutBits)));
-        const bool rf = avail < 32;
-        const uint64_t b2 = rf ? (buf | ((uint64_t)w << (32 - avail))) : buf;  // >= 32 valid bits
-        const int a2 = rf ? avail + 32 : avail;
-        if (rf) w = rd(wi++);
-        uint32_t sym = e & 0xffffu, l = (e >> 16) & 0xffu;
-        if (!l) {
-            // canonical search from the shortest length under this prefix; a
-            // corrupt stream still yields a symbol of this codebook (never
-            // code 0 unless the stream has unpredictable values)
-            l = e >> 24;
-            if (!l) l = kLutBits + 1;
-            for (; l <= (uint32_t)kMaxCodeLen; ++l) {
-                const uint32_t v = (uint32_t)(b2 >> (64 - l));
-                if (v - first_code[l] < cnt[l]) {
-                    const uint32_t idx = first_idx[l] + (v - first_code[l]);
-                    const uint32_t ti = idx - first_idx[kLutBits + 1];
-                    sym = ti < (uint32_t)kTailSyms ? __ldg(&t->tail[ti]) : cb_sym[s.cb_off + idx];
-                    break;
-                }
-            }
-            if (l > (uint32_t)kMaxCodeLen) {
-                sym = cb_sym[s.cb_off];
-                l = 1;  // corrupt stream: keep going, the result is garbage
-            }
-        }
-        buf = b2 << l;
-        avail = a2 - (int)l;
-        if (avail < kLutBits) {  // only after a long code taken without a refill
-            buf |= (uint64_t)w << (32 - avail);
-            avail += 32;
-            w = rd(wi++);
-        }
-        return sym;
-    };
-    if (s.run_n) {
-        // Runs expand to 2^k centre codes, clipped to the plane (a corrupt
-        // stream cannot write past it; every symbol yields at least one code,
-        // so the loop ends). Vector form: codes collect in a 128-bit shift
-        // register and leave as 16-byte stores; long runs store whole
-        // 8-code groups directly.
-        const uint32_t R = s.radius, base = s.run_base, J = s.run_n;
-        uint32_t D, LD;
-        run_geometry((uint32_t)plane, D, LD);
-        size_t j = 0;
-        if (plane % 8 == 0 && ((uintptr_t)dst & 15) == 0) {
-            // 8 staged codes in (s0, s1), slot i at bits 16i; n copies of a
-            // code enter with one masked OR, a full stage leaves as one store
-            uint4* d4 = reinterpret_cast<uint4*>(dst);
-            uint64_t s0 = 0, s1 = 0;
-            uint32_t ns = 0;
-            auto low = [](uint32_t b) -> uint64_t { return b >= 64 ? ~0ull : (1ull << b) - 1; };
-            auto flush = [&]() {
-                if (ns == 8) {
-                    d4[(j >> 3) - 1] =
-                        make_uint4((uint32_t)s0, (uint32_t)(s0 >> 32), (uint32_t)s1, (uint32_t)(s1 >> 32));
-                    s0 = s1 = 0;
-                    ns = 0;
-                }
-            };
-            auto put = [&](uint32_t v, uint32_t n) {  // n <= 8 - ns copies of v
-                const uint64_t p = (uint64_t)(v | (v << 16)) * 0x0000000100000001ull;
-                const uint32_t a = 16 * ns, b = 16 * (ns + n);
-                s0 |= p & (low(min(b, 64u)) & ~low(min(a, 64u)));
-                s1 |= p & (low(b > 64 ? b - 64 : 0) & ~low(a > 64 ? a - 64 : 0));
-                ns += n;
-                j += n;
-                flush();
-            };
-            auto put1 = [&](uint32_t v) {  // one code: a shift into its slot
-                if (ns < 4) s0 |= (uint64_t)v << (16 * ns);
-                else s1 |= (uint64_t)v << (16 * (ns - 4));
-                ++ns;
-                ++j;
-                flush();
-            };
-            const uint32_t r2 = R | (R << 16);
-            const uint4 rr = make_uint4(r2, r2, r2, r2);
-            while (j < plane) {
-                const uint32_t sym = next();
-                if (sym - base < J) {
-                    uint32_t n = (uint32_t)min((size_t)run_length(sym - base, D, LD), plane - j);
-                    if (ns) {
-                        const uint32_t k = min(n, 8u - ns);
-                        put(R, k);
-                        n -= k;
-                    }
-                    for (; n >= 8; n -= 8, j += 8) d4[j >> 3] = rr;
-                    if (n) put(R, n);
-                } else {
-                    put1(sym);
-                }
-            }
-        } else {
-            while (j < plane) {
-                const uint32_t sym = next();
-                if (sym - base < J) {
-                    const size_t n = min((size_t)run_length(sym - base, D, LD), plane - j);
-                    for (size_t i = 0; i < n; ++i) dst[j++] = (uint16_t)R;
-                } else {
-                    dst[j++] = (uint16_t)sym;
-                }
-            }
-        }
-    } else if (plane % 8 == 0 && ((uintptr_t)dst & 15) == 0) {
-        // 8 symbols per 16-byte store; all lanes decode in lockstep
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
-        for (size_t j = 0; j < plane / 8; ++j) {
-            uint4 v;
-            v.x = next();
-            v.x |= next() << 16;
-            v.y = next();
-            v.y |= next() << 16;
-            v.z = next();
-            v.z |= next() << 16;
-            v.w = next();
-            v.w |= next() << 16;
-            d4[j] = v;
-        }
-    } else {
-        for (size_t j = 0; j < plane; ++j) dst[j] = (uint16_t)next();
-    }
-}
-
-// Decode plane lz of chunk c of stream s (one group of W lanes, see
-// lanes_per_plane; Weissenberger & Schmidt, "Massively parallel Huffman
-// decoding on GPUs", ICPP 2018: speculative decoding from equal bit slices,
-// then resynchronisation). A group without a plane (active false) takes part
-// in the shuffles only. The plane's bits [b0, b1) are cut into W slices;
-// lane i decodes the codes that start in
-// its slice, beginning at the slice start. A lane whose start is not where
-// its left neighbour's last code ends decodes again from there, until no
-// start moves (lane i is exact after i rounds; codes resynchronise within a
-// few symbols, so one or two rounds are usual). An exclusive scan of the
-// lanes' code counts (a run symbol counts its run) then places each lane's
-// output. With run symbols the plane is first filled with the centre code,
-// so a lane writes only its literals. Output past the plane (a corrupt
-// stream) is dropped.
-__device__ void decode_plane_warp(const DecodeTables* __restrict__ t, const StreamDesc& s, uint32_t W, bool active,
-                                  uint32_t c, uint32_t lz,
-                                  const uint16_t* __restrict__ cb_sym, const uint32_t* __restrict__ sub_off,
-                                  const uint64_t* __restrict__ chunk_word_off, const uint32_t* __restrict__ payload,
-                                  uint16_t* __restrict__ codes)
-{
-    const uint32_t lane = threadIdx.x & (W - 1);
-    const uint32_t C = s.C, P = C * C;
-    uint16_t* dst = codes + s.code_off + (size_t)c * P * C + (size_t)lz * P;
-    const bool vec = P % 8 == 0 && ((uintptr_t)dst & 15) == 0;
-    const uint32_t R = s.radius, base = s.run_base, J = s.run_n;
-    auto fill = [&](uint16_t v) {
-        if (!active) return;
-        if (vec) {
-            const uint32_t v2 = (uint32_t)v | ((uint32_t)v << 16);
-            for (uint32_t j = lane; j < P / 8; j += W) reinterpret_cast<uint4*>(dst)[j] = make_uint4(v2, v2, v2, v2);
-        } else {
-            for (uint32_t j = lane; j < P; j += W) dst[j] = v;
+    const uint32_t nb = r1 - r0, L = (nb + W - 1) / W;
+    const uint32_t stop = r0 + min(nb, (lane + 1) * L);
+    uint32_t start = r0 + min(nb, lane * L), end = start, cnt = 0;
+    auto count = [&]() {
+        cnt = 0;
+        while (end < stop) {
+            uint32_t l, val;
+            bool run, late;
+            dc.symbol<SMEM>(peek(w, end), l, val, run, late);
+            cnt += run ? val : 1u;
+            end += l;
         }
     };
-    if (s.n_used == 1) {
-        // a lone run symbol means the plane is all centre codes
-        const uint16_t v0 = cb_sym[s.cb_off];
-        fill((uint32_t)v0 - base < J ? (uint16_t)R : v0);
-        return;
-    }
-    const uint64_t cw = chunk_word_off[s.chunk_base + c];
-    ChunkBits cb;
-    cb.in = payload + s.word_base + cw;
-    const uint32_t b0 = sub_off[s.sub_base + (size_t)c * C + lz];
-    const uint32_t b1 = lz + 1 < C ? sub_off[s.sub_base + (size_t)c * C + lz + 1]
-                                   : (uint32_t)(32 * (chunk_word_off[s.chunk_base + c + 1] - cw));
-    const uint32_t nb = active && b1 > b0 ? b1 - b0 : 0;
-    const uint32_t L = (nb + W - 1) / W;
-    const uint32_t stop = b0 + min(nb, (lane + 1) * L);
-    uint32_t D, LD;
-    run_geometry(P, D, LD);
-    uint32_t start = b0 + min(nb, lane * L), cnt = 0;
-    auto count = [&](uint32_t sym) { cnt += sym - base < J ? run_length(sym - base, D, LD) : 1u; };
-    uint32_t end = decode_range(t, s, cb_sym, cb, start, stop, count);
-    for (int round = 0; round < 32; ++round) {
+    count();
+    for (uint32_t round = 0; round < W; ++round) {
         uint32_t prev = __shfl_up_sync(0xffffffffu, end, 1, W);
-        if (lane == 0) prev = b0;
+        if (lane == 0) prev = r0;
         const bool moved = prev != start;
         if (!__any_sync(0xffffffffu, moved)) break;
         if (moved) {
-            start = prev;
-            cnt = 0;
-            end = decode_range(t, s, cb_sym, cb, start, stop, count);
+            start = end = prev;
+            count();
         }
     }
-    uint32_t q = group_scan(cnt, W, lane) - cnt;  // first output position
-    if (J) {
-        fill((uint16_t)R);
-        __syncwarp();
-        decode_range(t, s, cb_sym, cb, start, stop, [&](uint32_t sym) {
-            if (sym - base < J) {
-                q += run_length(sym - base, D, LD);
-            } else {
-                if (active && q < P) dst[q] = (uint16_t)sym;
-                ++q;
-            }
-        });
-    } else {
-        decode_range(t, s, cb_sym, cb, start, stop, [&](uint32_t sym) {
-            if (active && q < P) dst[q] = (uint16_t)sym;
-            ++q;
-        });
+    uint32_t q = group_scan(cnt, W, lane) - cnt;  // first code of this lane
+    while (start < stop) {
+        uint32_t l, val;
+        bool run, late;
+        dc.symbol<SMEM>(peek(w, start), l, val, run, late);
+        if (!run) put(q, val, late);
+        q += run ? val : 1u;
+        start += l;
     }
 }
 
-constexpr int kDecodeThreads = 256;  // 8 warps, each one plane
-constexpr int kDecodeSlices = 16;    // CTAs per work item (gridDim.y): short CTAs, every warp one plane
-constexpr uint32_t kSeqBits = 2048;  // mean payload bits per plane above which a stream decodes one thread per plane
+// Lanes per plane: as many as leave a lane about 32 codes.
+__device__ __forceinline__ uint32_t decode_lanes(uint32_t P)
+{
+    uint32_t W = 1;
+    while (W < 32 && 32 * W < P) W *= 2;
+    return W;
+}
 
-// Lanes decoding one plane: a warp for planes of 1024 codes and more, but
-// half a warp where a plane averages fewer than kHalfWarpBits payload bits:
-// each lane then takes twice the bits, and the resynchronisation and scans
-// cost half as much per symbol (512^3 bench stream, ~600 bits per plane:
-// 0.40 -> 0.34 ms; 8 lanes 0.40, 4 lanes 0.59).
+// One plane's place: its bits in the payload words from the 16-byte group it
+// starts in, and its codes.
+struct PlaneAt {
+    const uint32_t* src;
+    uint16_t* dst;
+    uint32_t r0, r1;
+};
+__device__ __forceinline__ PlaneAt plane_at(const StreamDesc& s, const uint32_t* __restrict__ chunks, uint32_t p,
+                                            bool active, const uint32_t* __restrict__ sub_off,
+                                            const uint64_t* __restrict__ chunk_word_off,
+                                            const uint32_t* __restrict__ payload, uint16_t* __restrict__ codes)
+{
+    const uint32_t C = s.C, P = C * C, pc = p / C, lz = p - pc * C, c = chunks[pc];
+    const uint64_t cw = chunk_word_off[s.chunk_base + c];
+    const uint32_t b0 = sub_off[s.sub_base + (size_t)c * C + lz];
+    const uint32_t b1 = lz + 1 < C ? sub_off[s.sub_base + (size_t)c * C + lz + 1]
+                                   : (uint32_t)(32 * (chunk_word_off[s.chunk_base + c + 1] - cw));
+    const uint64_t w0 = s.word_base + cw + (b0 >> 5);
+    PlaneAt a;
+    a.src = payload + (w0 & ~3ull);
+    a.dst = codes + s.code_off + (size_t)c * P * C + (size_t)lz * P;
+    a.r0 = ((uint32_t)(w0 & 3) << 5) + (b0 & 31);
+    a.r1 = a.r0 + (active && s.n_used != 1 && b1 > b0 ? b1 - b0 : 0u);  // a lone symbol has no bits
+    return a;
+}
+
+// Half a warp decodes a plane of a stream with fewer payload bits per plane
+// than this on average, in launches of at least kHalfWarpItems items: each
+// lane then takes twice the bits, and the rounds and scans cost half as much
+// per symbol (512^3 f32 at 1e-3, ~600 bits per plane, the finest level's
+// halves: 0.18 + 0.14 -> 0.16 + 0.12 ms). Two planes of 1024 codes do not fit
+// the warp's buffer: centre codes go to global memory first and literals over
+// them. Smaller launches are bound by latency and take all 32 lanes.
 constexpr uint32_t kHalfWarpBits = 2048;
-__device__ __forceinline__ uint32_t decode_group(const StreamDesc& s)
+constexpr int kHalfWarpItems = 128;
+
+// A code without a literal: the centre code; a lone symbol that is not a run
+// fills the plane itself.
+__device__ __forceinline__ uint32_t fill_code(const StreamDesc& s, const uint16_t* __restrict__ syms)
 {
-    const uint32_t W = lanes_per_plane(s.C * s.C);
-    const uint64_t planes = (uint64_t)s.nchunks * s.C;
-    return W == 32 && 32 * (s.word_cap - 4) < (uint64_t)kHalfWarpBits * planes ? 16u : W;
+    return s.n_used == 1 && (uint32_t)syms[0] - s.run_base >= s.run_n ? (uint32_t)syms[0] : s.radius;
 }
 
-// A stream whose planes average more than seq_bits payload bits, with enough
-// planes to fill the device one thread per plane, is decoded one thread per
-// plane; sparser or smaller streams a lane group per plane (decode_group: the
-// group decodes each symbol about three times, a thread once but with the
-// full serial chain).
-constexpr uint64_t kSeqMinPlanes = 16384;
-constexpr int kSeqMinItems = 128;  // smaller launches (single requests) are latency-bound: warps only
-__device__ __forceinline__ bool decode_sequential(const StreamDesc& s, uint32_t seq_bits)
+// Planes too large for the shared buffers: everything through L1, centre codes
+// stored first, literals over them.
+__device__ __forceinline__ void decode_direct(const StreamDesc& s, const DecodeTables* __restrict__ t, uint32_t W,
+                                              const uint32_t* __restrict__ chunks, uint32_t np, uint32_t first,
+                                              uint32_t nwarps, const uint16_t* __restrict__ cb_sym,
+                                              const uint32_t* __restrict__ sub_off,
+                                              const uint64_t* __restrict__ chunk_word_off,
+                                              const uint32_t* __restrict__ payload, uint16_t* __restrict__ codes)
 {
-    const uint64_t planes = (uint64_t)s.nchunks * s.C;
-    return planes >= kSeqMinPlanes && 32 * (s.word_cap - 4) > (uint64_t)seq_bits * planes;
+    const uint32_t G = 32 / W, lane = threadIdx.x & (W - 1), gi = (threadIdx.x & 31) / W, P = s.C * s.C;
+    const uint16_t* __restrict__ syms = cb_sym + s.cb_off;
+    const uint32_t fill = fill_code(s, syms);
+    const bool by_index = t->by_index;
+    const DecodeCtx dc{t->lut, t};
+    for (uint32_t base = first * G; base < np; base += nwarps * G) {
+        const bool active = base + gi < np;
+        const PlaneAt a = plane_at(s, chunks, active ? base + gi : base, active, sub_off, chunk_word_off, payload, codes);
+        if (active) {
+            if (P % 8 == 0 && ((uintptr_t)a.dst & 15) == 0) {
+                const uint32_t f2 = fill * 0x10001u;
+                for (uint32_t k = lane; k < P / 8; k += W)
+                    reinterpret_cast<uint4*>(a.dst)[k] = make_uint4(f2, f2, f2, f2);
+            } else {
+                for (uint32_t k = lane; k < P; k += W) a.dst[k] = (uint16_t)fill;
+            }
+        }
+        __syncwarp();
+        decode_plane<false>(dc, [&](uint32_t i) { return __ldg(a.src + i); }, a.r0, a.r1, W, lane,
+                            [&](uint32_t q, uint32_t val, bool late) {
+                                if (q < P) a.dst[q] = late || by_index ? __ldg(syms + val) : (uint16_t)val;
+                            });
+    }
 }
 
-// Planes of the listed chunks; the tables of stream i at tabs[i]. Warp mode:
-// CTA (x, y) takes 8 planes of item x; sequential mode: CTA (x, 0) takes all
-// of them, one per thread (at most kDecodeThreads).
-__global__ void __launch_bounds__(kDecodeThreads, 5) k_decode(const CtaWork* __restrict__ work,
+// Payload and table in shared memory, and the codes too where the warp's
+// planes fit its buffer: then only final values are stored, each once.
+__device__ __forceinline__ void decode_buffered(DecodeSmem& sm, const StreamDesc& s,
+                                                const DecodeTables* __restrict__ t, uint32_t W,
+                                                const uint32_t* __restrict__ chunks, uint32_t np, uint32_t first,
+                                                uint32_t nwarps, const uint16_t* __restrict__ cb_sym,
+                                                const uint32_t* __restrict__ sub_off,
+                                                const uint64_t* __restrict__ chunk_word_off,
+                                                const uint32_t* __restrict__ payload, uint16_t* __restrict__ codes)
+{
+    const uint32_t P = s.C * s.C, G = 32 / W, wid = threadIdx.x >> 5, all = threadIdx.x & 31;
+    if (first * G >= np) return;  // uniform per warp; nothing below waits for the other warps
+    const bool direct = G * P > kMaxPlane;
+    const uint32_t lane = all & (W - 1), gi = all / W;
+    const uint16_t* __restrict__ syms = cb_sym + s.cb_off;
+    const bool by_index = t->by_index;
+    const uint32_t f2 = (by_index && !direct ? kNoIndex : fill_code(s, syms)) * 0x10001u;
+    const uint4 f4 = make_uint4(f2, f2, f2, f2);
+    const uint32_t Pc = (P + 7) & ~7u;      // codes of a group's share of the buffer (G * Pc <= kMaxPlane)
+    const uint32_t cap = kStageWords / G;   // payload words of it
+    uint4* const out = sm.out[wid] + gi * (Pc / 8);
+    uint16_t* const out16 = reinterpret_cast<uint16_t*>(out);
+    uint4* const stage = sm.stage[wid] + gi * (cap / 4);
+    uint32_t* const late = sm.late[wid];
+    if (!direct) {
+        for (uint32_t k = all; k < kMaxPlane / 8; k += 32) sm.out[wid][k] = f4;
+        late[all] = 0;
+    }
+    __syncwarp();
+    const DecodeCtx dc{sm.lut, t};
+    for (uint32_t base = first * G; base < np; base += nwarps * G) {
+        const bool active = base + gi < np;
+        const PlaneAt a = plane_at(s, chunks, active ? base + gi : base, active, sub_off, chunk_word_off, payload, codes);
+        bool any_late = false;
+        auto put = [&](uint32_t q, uint32_t val, bool lt) {
+            if (q >= P) return;  // corrupt stream
+            if (direct) {
+                a.dst[q] = lt || by_index ? __ldg(syms + val) : (uint16_t)val;
+                return;
+            }
+            out16[q] = (uint16_t)val;
+            if (lt && !by_index) {
+                const uint32_t x = gi * Pc + q;
+                atomicOr(&late[x >> 5], 1u << (x & 31));
+                any_late = true;
+            }
+        };
+        const uint32_t nw = a.r1 > a.r0 ? ((a.r1 + 31) >> 5) + 2 : 0u;
+        if (direct) {
+            if (active)
+                for (uint32_t k = lane; k < P / 8; k += W) reinterpret_cast<uint4*>(a.dst)[k] = f4;
+            __syncwarp();
+        }
+        if (__all_sync(0xffffffffu, nw <= cap)) {
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(stage);
+            for (uint32_t k = lane; k < (nw + 3) / 4; k += W)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(at + k * 16), "l"(a.src + 4 * k)
+                             : "memory");
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            const uint32_t* const sw = reinterpret_cast<const uint32_t*>(stage);
+            decode_plane<true>(dc, [&](uint32_t i) { return sw[i]; }, a.r0, a.r1, W, lane, put);
+        } else {
+            decode_plane<true>(dc, [&](uint32_t i) { return __ldg(a.src + i); }, a.r0, a.r1, W, lane, put);
+        }
+        __syncwarp();
+        if (direct) continue;
+        any_late = __any_sync(0xffffffffu, any_late);
+        // the planes to global memory, the buffer back to its empty state
+        const bool vec = P % 8 == 0 && ((uintptr_t)a.dst & 15) == 0;
+        for (uint32_t k = lane; k < Pc / 8; k += W) {
+            const uint4 v = out[k];
+            out[k] = f4;
+            if (!active) continue;
+            uint32_t x[4] = {v.x, v.y, v.z, v.w};
+            if (by_index) {
+                auto sym = [&](uint32_t i) -> uint32_t { return i < s.n_used ? __ldg(syms + i) : s.radius; };
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = sym(x[j] & 0xffffu) | sym(x[j] >> 16) << 16;
+            } else if (any_late) {
+                const uint32_t m = late[(gi * Pc + 8 * k) >> 5] >> ((gi * Pc + 8 * k) & 31) & 0xffu;
+                if (m)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (m >> (2 * j) & 1u) x[j] = (x[j] & 0xffff0000u) | __ldg(syms + (x[j] & 0xffffu));
+                        if (m >> (2 * j + 1) & 1u) x[j] = (x[j] & 0xffffu) | (uint32_t)__ldg(syms + (x[j] >> 16)) << 16;
+                    }
+            }
+            if (vec) {
+                *reinterpret_cast<uint4*>(a.dst + 8 * k) = make_uint4(x[0], x[1], x[2], x[3]);
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j)
+                    if (8 * k + j < P) a.dst[8 * k + j] = (uint16_t)(x[j >> 1] >> (16 * (j & 1)));
+            }
+        }
+        __syncwarp();
+        if (any_late) late[all] = 0;
+        __syncwarp();
+    }
+}
+
+// The stream's table into shared memory (the whole CTA; a barrier before the
+// old one is overwritten and one after).
+__device__ __forceinline__ void load_table(DecodeSmem& sm, const DecodeTables* __restrict__ t)
+{
+    __syncthreads();
+    const uint4* __restrict__ src = reinterpret_cast<const uint4*>(t->lut);
+    for (uint32_t i = threadIdx.x; i < (1u << kLutBits) / 4; i += kDecodeThreads)
+        reinterpret_cast<uint4*>(sm.lut)[i] = __ldg(src + i);
+    __syncthreads();
+}
+
+// CTAs that share a work item: a plane per warp, down to a few per warp in
+// the largest launches. Short CTAs balance better than they pay for loading
+// the table (finest level's halves, 448 items, 512^3 f32 at 1e-4: 0.63 + 0.51
+// ms with one CTA an item, 0.56 + 0.41 with four, 0.50 + 0.32 with eight).
+__host__ __device__ inline uint32_t decode_slices(uint32_t nwork)
+{
+    uint32_t S = 16;
+    while (S > 1 && (uint64_t)nwork * S > 148 * 48) S /= 2;
+    return S;
+}
+
+// Planes of the listed chunks: CTA (x, y) takes the planes of item x that
+// fall to its warps of the item's gridDim.y * kDecodeWarps; the tables of
+// stream i at tabs[i].
+__global__ void __launch_bounds__(kDecodeThreads) k_decode(const CtaWork* __restrict__ work,
                                                            const uint32_t* __restrict__ chunk_ids,
                                                            const StreamDesc* __restrict__ sd,
                                                            const DecodeTables* __restrict__ tabs,
@@ -1108,69 +1114,64 @@ __global__ void __launch_bounds__(kDecodeThreads, 5) k_decode(const CtaWork* __r
                                                            const uint32_t* __restrict__ sub_off,
                                                            const uint64_t* __restrict__ chunk_word_off,
                                                            const uint32_t* __restrict__ payload,
-                                                           uint16_t* __restrict__ codes, uint32_t seq_bits)
+                                                           uint16_t* __restrict__ codes, bool halves)
 {
+    extern __shared__ __align__(16) uint8_t decode_smem[];
+    DecodeSmem& sm = *reinterpret_cast<DecodeSmem*>(decode_smem);
     const CtaWork w = work[blockIdx.x];
     const StreamDesc s = sd[w.stream];
-    if (decode_sequential(s, seq_bits)) {
-        const uint32_t t = threadIdx.x;
-        if (blockIdx.y == 0 && t < w.count * s.C)
-            decode_plane_seq(tabs + w.stream, s, chunk_ids[w.first + t / s.C], t % s.C, cb_sym, sub_off,
-                             chunk_word_off, payload, codes);
+    const uint32_t P = s.C * s.C, np = w.count * s.C;
+    uint32_t W = decode_lanes(P);
+    if (halves && P == kMaxPlane && s.code_off % 8 == 0 &&
+        32 * (s.word_cap - 4) < (uint64_t)kHalfWarpBits * s.nchunks * s.C)
+        W = 16;
+    if (blockIdx.y * kDecodeWarps * (32 / W) >= np) return;  // uniform per block
+    const uint32_t first = blockIdx.y * kDecodeWarps + (threadIdx.x >> 5), nwarps = gridDim.y * kDecodeWarps;
+    if (P > kMaxPlane) {
+        decode_direct(s, tabs + w.stream, W, chunk_ids + w.first, np, first, nwarps, cb_sym, sub_off, chunk_word_off,
+                      payload, codes);
         return;
     }
-    const uint32_t W = decode_group(s), np = w.count * s.C;
-    STZ_GROUP_PLANES(np, W)
-    {
-        STZ_GROUP_PLANE(np, W);
-        decode_plane_warp(tabs + w.stream, s, W, active, chunk_ids[w.first + pe / s.C], pe % s.C, cb_sym, sub_off,
-                          chunk_word_off, payload, codes);
-    }
+    load_table(sm, tabs + w.stream);
+    decode_buffered(sm, s, tabs + w.stream, W, chunk_ids + w.first, np, first, nwarps, cb_sym, sub_off, chunk_word_off,
+                    payload, codes);
 }
 
 // Persistent variant: a fixed grid walks the work list of a batch held in
-// device memory (BatchHdr at meta), so one captured launch serves any batch;
-// each warp-decoded item is cut into kDecodeSlices slices of 8 planes.
-__global__ void __launch_bounds__(kDecodeThreads) k_decode_dyn(const uint8_t* __restrict__ meta,
+// device memory (BatchHdr at meta), so one captured launch serves any batch.
+__global__ void __launch_bounds__(kDecodeThreads, 3) k_decode_dyn(const uint8_t* __restrict__ meta,
                                                                const StreamDesc* __restrict__ sd,
                                                                const DecodeTables* __restrict__ tabs,
                                                                const uint16_t* __restrict__ cb_sym,
                                                                const uint32_t* __restrict__ sub_off,
                                                                const uint64_t* __restrict__ chunk_word_off,
                                                                const uint32_t* __restrict__ payload,
-                                                               uint16_t* __restrict__ codes, uint32_t seq_bits)
+                                                               uint16_t* __restrict__ codes)
 {
+    extern __shared__ __align__(16) uint8_t decode_smem[];
+    DecodeSmem& sm = *reinterpret_cast<DecodeSmem*>(decode_smem);
     const BatchHdr* h = reinterpret_cast<const BatchHdr*>(meta);
     const uint32_t n = h->n_work;
+    if (n == 0) return;
     const CtaWork* __restrict__ work = reinterpret_cast<const CtaWork*>(meta + h->o_work);
     const uint32_t* __restrict__ chunk_ids = reinterpret_cast<const uint32_t*>(meta + h->o_ids);
-    const uint32_t nw = blockDim.x >> 5, S = kDecodeSlices;
-    // In a batch of at least kSeqMinItems items, dense streams decode one
-    // thread per plane (as k_decode does for large launches): a CTA takes
-    // whole items, striding over the items so every CTA gets some.
-    const uint32_t sb = n >= (uint32_t)kSeqMinItems ? seq_bits : 0xffffffffu;
-    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-        const CtaWork w = work[i];
+    const uint32_t S = decode_slices(n);
+    uint32_t loaded = 0xffffffffu;  // stream whose table is in shared memory
+    for (uint32_t i = blockIdx.x; i < n * S; i += gridDim.x) {
+        const CtaWork w = work[i / S];
         const StreamDesc s = sd[w.stream];
-        if (!decode_sequential(s, sb)) continue;  // uniform per block
-        const uint32_t t = threadIdx.x;
-        if (t < w.count * s.C)
-            decode_plane_seq(tabs + w.stream, s, chunk_ids[w.first + t / s.C], t % s.C, cb_sym, sub_off,
-                             chunk_word_off, payload, codes);
-    }
-    // the other items a warp per plane, kDecodeSlices slices per item
-    for (uint32_t u = blockIdx.x; u < n * S; u += gridDim.x) {
-        const CtaWork w = work[u / S];
-        const StreamDesc s = sd[w.stream];
-        if (decode_sequential(s, sb)) continue;  // uniform per block
-        const uint32_t W = decode_group(s), G = 32 / W, np = w.count * s.C;
-        for (uint32_t base = ((u % S) * nw + (threadIdx.x >> 5)) * G; base < np; base += nw * S * G) {
-            const uint32_t p = base + (threadIdx.x & 31) / W;
-            const bool active = p < np;
-            const uint32_t pe = active ? p : base;
-            decode_plane_warp(tabs + w.stream, s, W, active, chunk_ids[w.first + pe / s.C], pe % s.C, cb_sym, sub_off,
-                              chunk_word_off, payload, codes);
+        const uint32_t P = s.C * s.C, W = decode_lanes(P), np = w.count * s.C;
+        if (i % S * kDecodeWarps * (32 / W) >= np) continue;  // uniform per block
+        const uint32_t first = i % S * kDecodeWarps + (threadIdx.x >> 5);
+        if (P > kMaxPlane) {
+            decode_direct(s, tabs + w.stream, W, chunk_ids + w.first, np, first, S * kDecodeWarps, cb_sym, sub_off,
+                          chunk_word_off, payload, codes);
+            continue;
         }
+        if (w.stream != loaded) load_table(sm, tabs + w.stream);
+        loaded = w.stream;
+        decode_buffered(sm, s, tabs + w.stream, W, chunk_ids + w.first, np, first, S * kDecodeWarps, cb_sym, sub_off,
+                        chunk_word_off, payload, codes);
     }
 }
 
@@ -1308,28 +1309,20 @@ void launch_decode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, co
                    const uint16_t* cb_sym, const void* tables, const uint32_t* sub_off, const uint64_t* chunk_word_off,
                    const uint32_t* payload, uint16_t* codes, cudaStream_t st)
 {
-    if (nwork)
-        k_decode<<<dim3(nwork, kDecodeSlices), kDecodeThreads, 0, st>>>(
-            work, chunk_ids, sd, static_cast<const DecodeTables*>(tables), cb_sym, sub_off, chunk_word_off, payload,
-            codes, nwork >= kSeqMinItems ? decode_seq_bits() : 0xffffffffu);
+    if (!nwork) return;
+    cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecodeSmem));
+    const DecodeTables* t = static_cast<const DecodeTables*>(tables);
+    k_decode<<<dim3(nwork, decode_slices((uint32_t)nwork)), kDecodeThreads, sizeof(DecodeSmem), st>>>(
+        work, chunk_ids, sd, t, cb_sym, sub_off, chunk_word_off, payload, codes, nwork >= kHalfWarpItems);
 }
 
 size_t decode_tables_bytes() { return sizeof(DecodeTables); }
-
-uint32_t decode_seq_bits()
-{
-    static const uint32_t v = [] {
-        const char* e = std::getenv("STZ_DECODE_SEQ_BITS");
-        return e ? (uint32_t)std::strtoul(e, nullptr, 10) : kSeqBits;
-    }();
-    return v;
-}
 
 void launch_build_tables(const StreamDesc* sd, int nstreams, const uint16_t* cb_sym, const uint8_t* cb_len,
                          void* tables, cudaStream_t st)
 {
     if (nstreams > 0)
-        k_build_tables<<<nstreams, 256, 0, st>>>(sd, cb_sym, cb_len, static_cast<DecodeTables*>(tables));
+        k_build_tables<<<nstreams, kBuildThreads, 0, st>>>(sd, cb_sym, cb_len, static_cast<DecodeTables*>(tables));
 }
 
 template <typename T>
@@ -1350,8 +1343,9 @@ void launch_decode_dyn(int grid, const uint8_t* meta, const StreamDesc* sd, cons
                        const void* tables, const uint32_t* sub_off, const uint64_t* chunk_word_off,
                        const uint32_t* payload, uint16_t* codes, cudaStream_t st)
 {
-    k_decode_dyn<<<grid, kDecodeThreads, 0, st>>>(meta, sd, static_cast<const DecodeTables*>(tables), cb_sym, sub_off,
-                                                  chunk_word_off, payload, codes, decode_seq_bits());
+    cudaFuncSetAttribute(k_decode_dyn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecodeSmem));
+    k_decode_dyn<<<grid, kDecodeThreads, sizeof(DecodeSmem), st>>>(meta, sd, static_cast<const DecodeTables*>(tables), cb_sym, sub_off,
+                                                  chunk_word_off, payload, codes);
 }
 
 template <typename T>

@@ -62,11 +62,6 @@ void launch_decode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, co
 // Decode tables of every stream (read by the decoders): decode_tables_bytes()
 // each, stream i at byte i * decode_tables_bytes() of `tables`.
 size_t decode_tables_bytes();
-// Mean payload bits per plane above which launch_decode decodes a stream one
-// thread per plane instead of a lane group per plane, in launches of at least 128
-// work items and for streams of at least 16384 planes (STZ_DECODE_SEQ_BITS
-// overrides the built-in 2048).
-uint32_t decode_seq_bits();
 void launch_build_tables(const StreamDesc* sd, int nstreams, const uint16_t* cb_sym, const uint8_t* cb_len,
                          void* tables, cudaStream_t st);
 // The payload words of streams [s0, s1) back to back in stream order into dst
