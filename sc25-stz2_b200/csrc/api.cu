@@ -202,7 +202,7 @@ int pool_threads(int requested)
 }
 
 namespace {
-constexpr size_t kXferChunk = 8ull << 20;
+constexpr size_t kXferChunk = 16ull << 20;
 
 bool host_pinned(const void* p)
 {
@@ -214,14 +214,14 @@ bool host_pinned(const void* p)
     return a.type == cudaMemoryTypeHost;
 }
 
-// copy of n bytes on the pool, in pieces of at least 512 KiB
+// memcpy of n bytes on the pool, in pieces of at least 1 MiB
 void pool_copy(ThreadPool& pool, void* dst, const void* src, size_t n)
 {
-    const size_t parts = std::max<size_t>(1, std::min<size_t>((size_t)pool.size(), n >> 19));
+    const size_t parts = std::max<size_t>(1, std::min<size_t>((size_t)pool.size(), n >> 20));
     const size_t per = (n + parts - 1) / parts;
     pool.parallel_for(parts, [&](size_t i) {
         const size_t a = i * per, b = std::min(n, a + per);
-        if (a < b) stream_copy((uint8_t*)dst + a, (const uint8_t*)src + a, b - a);
+        if (a < b) std::memcpy((uint8_t*)dst + a, (const uint8_t*)src + a, b - a);
     });
 }
 
@@ -817,13 +817,12 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     // finest streams', the largest, first)
     auto build_header = [&](size_t s) {
         const StreamDesc& d = sd[s];
-        build_stream_header(parts[s], ctx->arena, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
-                            unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
-                            h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
-                            (int)d.C);
+        append_stream_header(parts[s].hdr, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
+                             unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
+                             h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
+                             (int)d.C);
     };
-    ctx->arena.reset();
-    ContainerWriter cw(h, parts, *ctx->pool, ctx->arena);
+    ContainerWriter cw(h, parts, *ctx->pool);
     std::atomic<int> ev_err{0};
     // a group's copy seen complete once: later frames of the group make no
     // CUDA call (concurrent calls from the pool's threads serialize in the
@@ -941,8 +940,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
     const int nstreams = 7 * kmax;
     p.kmax = kmax;
     p.sd.assign(nstreams, StreamDesc{});
-    p.hdr.resize(nstreams);
-    ctx->arena.reset();
+    p.hdr.assign(nstreams, StreamHeader{});
     p.unpred_prefix.assign(nstreams, {});
     std::atomic<int> bad{0};
     std::vector<const char*> why(nstreams, nullptr);
@@ -952,10 +950,10 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         const int k = (int)i / 7 + 1, b = (int)i % 7;
         const LevelDir& L = ps.lv[k];
         const StreamDir& d = L.s[b];
-        ArenaBlock raw;
+        std::vector<uint8_t> raw(d.hdr_raw);
         const int nch = (L.dx / L.C) * (L.dy / L.C) * (L.dz / L.C);
-        if (!raw.take(ctx->arena, d.hdr_raw) || !decode_frame(bytes + d.data_off, d.hdr_stored, d.hdr_raw, raw.p)) bad = 1;
-        else if (!parse_stream_header(raw.p, d.hdr_raw, nch, L.C, elem, ps.version, p.hdr[i])) bad = 2;
+        if (!decode_frame(bytes + d.data_off, d.hdr_stored, d.hdr_raw, raw.data())) bad = 1;
+        else if (!parse_stream_header(raw.data(), raw.size(), nch, L.C, elem, ps.version, p.hdr[i])) bad = 2;
         else why[i] = check_stream(h, L, d, p.hdr[i], p.unpred_prefix[i]);
     });
     if (bad) STZ_FAIL(STZ_ERR_FORMAT, bad == 1 ? "stream header frame does not decode" : "bad stream header");
@@ -1012,9 +1010,9 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         const StreamDesc& d = p.sd[i];
         std::memcpy(hs + o_sym + 2 * (size_t)d.cb_off, H.sym.data(), 2 * H.sym.size());
         std::memcpy(hs + o_len + d.cb_off, H.len.data(), H.len.size());
-        stream_copy(hs + o_sub + 4 * d.sub_base, H.sub_off.data(), 4 * H.sub_off.size());
-        stream_copy(hs + o_ch + 8 * d.chunk_base, H.chunk_word_off.data(), 8 * H.chunk_word_off.size());
-        if (H.n_unpred) stream_copy(hs + o_ul + p.ulist_off[i] * elem, H.unpred.data(), H.unpred.size());
+        std::memcpy(hs + o_sub + 4 * d.sub_base, H.sub_off.data(), 4 * H.sub_off.size());
+        std::memcpy(hs + o_ch + 8 * d.chunk_base, H.chunk_word_off.data(), 8 * H.chunk_word_off.size());
+        if (H.n_unpred) std::memcpy(hs + o_ul + p.ulist_off[i] * elem, H.unpred.data(), H.unpred.size());
     });
     lap.mark("layout + tables");
     // payload frames straight into the staging buffer
@@ -1107,8 +1105,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         }
         ctx->pool->parallel_for(bjobs.size(), [&](size_t i) {
             const Job& J = jobs[bjobs[i]];
-            if (J.stored == J.raw) stream_copy(J.dst, J.src, J.raw);
-            else if (!decode_frame(J.src, J.stored, J.raw, J.dst)) bad = 3;
+            if (!decode_frame(J.src, J.stored, J.raw, J.dst)) bad = 3;
         });
         if (bad) {
             sync_both();

@@ -128,14 +128,6 @@ struct Prepared {
     LearnedModel* d_models = nullptr;  // per level k (index k), when the stream has learned corrections
     void* d_tables = nullptr;          // decode tables per stream (launch_build_tables)
     bool base_valid = false;  // *base holds the decoded base grid (level K-2 output) for box queries
-    std::vector<StreamHeader>* hdr_home = nullptr;  // where a one-off decode's headers go back to (their memory is kept)
-    Prepared() = default;
-    Prepared(const Prepared&) = delete;
-    Prepared& operator=(const Prepared&) = delete;
-    ~Prepared()
-    {
-        if (hdr_home) hdr_home->swap(hdr);
-    }
 };
 
 // Where the level kernels evaluate the learned network: block-wide on the
@@ -269,14 +261,8 @@ struct stz_context {
     stz::PinBuf h_xfer[2];  // staging chunks of host <-> device copies of pageable caller buffers
     // device buffers lent to one-off decodes
     stz::DevBuf p_stage, p_coarsest, p_base;
-    // host memory kept between calls: frames and headers of a call, and the
-    // parsed headers of one-off decodes
-    stz::HostArena arena;
-    std::vector<stz::StreamHeader> hdr_scratch;
     void borrow(stz::Prepared& p)
     {
-        p.hdr.swap(hdr_scratch);
-        p.hdr_home = &hdr_scratch;
         p.stage = &p_stage;
         p.coarsest = &p_coarsest;
         p.base = &p_base;
