@@ -202,7 +202,7 @@ int pool_threads(int requested)
 }
 
 namespace {
-constexpr size_t kXferChunk = 16ull << 20;
+constexpr size_t kXferChunk = 8ull << 20;
 
 bool host_pinned(const void* p)
 {
@@ -214,14 +214,16 @@ bool host_pinned(const void* p)
     return a.type == cudaMemoryTypeHost;
 }
 
-// memcpy of n bytes on the pool, in pieces of at least 1 MiB
-void pool_copy(ThreadPool& pool, void* dst, const void* src, size_t n)
+// copy of n bytes on the pool, in pieces of at least 512 KiB; flush: src is
+// staging that a DMA writes next
+void pool_copy(ThreadPool& pool, void* dst, const void* src, size_t n, bool flush = false)
 {
-    const size_t parts = std::max<size_t>(1, std::min<size_t>((size_t)pool.size(), n >> 20));
+    const size_t parts = std::max<size_t>(1, std::min<size_t>((size_t)pool.size(), n >> 19));
     const size_t per = (n + parts - 1) / parts;
     pool.parallel_for(parts, [&](size_t i) {
         const size_t a = i * per, b = std::min(n, a + per);
-        if (a < b) std::memcpy((uint8_t*)dst + a, (const uint8_t*)src + a, b - a);
+        if (a < b) stream_copy((uint8_t*)dst + a, (const uint8_t*)src + a, b - a);
+        if (a < b && flush) flush_lines((const uint8_t*)src + a, b - a);
     });
 }
 
@@ -256,15 +258,19 @@ stz_status copy_to_host(stz_context* ctx, void* dst, const void* src_dev, size_t
         STZ_CUDA(cudaStreamSynchronize(st));
         return STZ_OK;
     }
+    // a third of the buffer a time: fresh pages of the caller's buffer fault
+    // and clear 2 MB at a time, and small chunks hold too few of them for all
+    // threads
+    const size_t chunk = std::min<size_t>(4 * kXferChunk, std::max(kXferChunk, (n / 3 + kXferChunk - 1) & ~(kXferChunk - 1)));
     XferEvents ev;
     DrainOnExit drain{st};
     for (int b = 0; b < 2; ++b) {
-        STZ_CUDA(ctx->h_xfer[b].ensure(kXferChunk));
+        STZ_CUDA(ctx->h_xfer[b].ensure(chunk));
         STZ_CUDA(cudaEventCreateWithFlags(&ev.e[b], cudaEventDisableTiming));
     }
-    const size_t nch = (n + kXferChunk - 1) / kXferChunk;
+    const size_t nch = (n + chunk - 1) / chunk;
     auto issue = [&](size_t i) -> cudaError_t {
-        const size_t a = i * kXferChunk, len = std::min(kXferChunk, n - a);
+        const size_t a = i * chunk, len = std::min(chunk, n - a);
         cudaError_t e = cudaMemcpyAsync(ctx->h_xfer[i & 1].p, (const uint8_t*)src_dev + a, len, cudaMemcpyDeviceToHost, st);
         return e == cudaSuccess ? cudaEventRecord(ev.e[i & 1], st) : e;
     };
@@ -272,8 +278,8 @@ stz_status copy_to_host(stz_context* ctx, void* dst, const void* src_dev, size_t
     for (size_t i = 0; i < nch; ++i) {
         if (i + 1 < nch) STZ_CUDA(issue(i + 1));  // into the other chunk, free since chunk i - 1 was copied out
         STZ_CUDA(cudaEventSynchronize(ev.e[i & 1]));
-        const size_t a = i * kXferChunk;
-        pool_copy(*ctx->pool, (uint8_t*)dst + a, ctx->h_xfer[i & 1].p, std::min(kXferChunk, n - a));
+        const size_t a = i * chunk;
+        pool_copy(*ctx->pool, (uint8_t*)dst + a, ctx->h_xfer[i & 1].p, std::min(chunk, n - a), true);
     }
     drain.done = true;  // every DMA was waited for above
     return STZ_OK;
@@ -604,13 +610,10 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     // ev.e[gi]: group gi's words are on the host; ev.e[ngroups + gi]: its
     // encode is done; then the named events below. The copies run on the
     // context's copy stream, so group gi's copy overlaps group gi + 1's
-    // encode. The pool's threads wait on the copy events ev.e[0, ngroups)
-    // while others compress frames: those waits block instead of spinning on
-    // a core.
+    // encode.
     enum { EvUp, EvLevels, EvCounts, EvBooks, EvInfo, EvScan, EvTables, EvUnpred, EvNamed };
     ev.e.assign(2 * ngroups + EvNamed, nullptr);
-    for (size_t i = 0; i < ev.e.size(); ++i)
-        STZ_CUDA(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming | (i < ngroups ? cudaEventBlockingSync : 0)));
+    for (size_t i = 0; i < ev.e.size(); ++i) STZ_CUDA(cudaEventCreateWithFlags(&ev.e[i], cudaEventDisableTiming));
     cudaEvent_t* named = ev.e.data() + 2 * ngroups;
     STZ_CUDA(cudaEventRecord(named[EvUp], sc));
     STZ_CUDA(cudaEventRecord(named[EvLevels], st));
@@ -671,6 +674,18 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaStreamWaitEvent(sc, named[EvBooks], 0));
     STZ_CUDA(cudaMemcpyAsync(hb, dbooks, (size_t)nstreams * sizeof(CodebookInfo), cudaMemcpyDeviceToHost, sc));
     STZ_CUDA(cudaEventRecord(named[EvInfo], sc));
+    // while the device works: what the pool read of the last call's tables and
+    // payload leaves the caches before this call's copies arrive there
+    {
+        const size_t piece = 256 << 10, a = (ctx->io_read + piece - 1) / piece, b = (ctx->payload_read + piece - 1) / piece;
+        ctx->pool->parallel_for(a + b, [&](size_t i) {
+            if (i < a) flush_lines(ctx->h_io.as<uint8_t>() + i * piece, std::min(piece, ctx->io_read - i * piece));
+            else
+                flush_lines(ctx->h_payload.as<uint8_t>() + (i - a) * piece,
+                            std::min(piece, ctx->payload_read - (i - a) * piece));
+        });
+        ctx->io_read = ctx->payload_read = 0;
+    }
     STZ_CUDA(cudaEventSynchronize(named[EvCounts]));
     std::vector<T> coarsest(n0);
     std::memcpy(coarsest.data(), ctx->h_small.as<uint8_t>() + 64, n0 * elem);
@@ -693,6 +708,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     const size_t t_sub = align256(t_choff + g.total_chunk_slots * 8);
     const size_t t_ul = align256(t_sub + g.total_sub * 4), t_bytes = align256(t_ul + total_unpred * elem);
     STZ_CUDA(ctx->h_io.ensure(t_bytes));
+    ctx->io_read = t_bytes;
     uint8_t* ht = ctx->h_io.as<uint8_t>();
     if (!uwork.empty()) {
         cudaStream_t su = ctx->st_side;
@@ -749,6 +765,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         packed_total += words[s];
     }
     STZ_CUDA(ctx->h_payload.ensure(std::max<uint64_t>(packed_total, 1) * 4));
+    ctx->payload_read = packed_total * 4;
     struct Piece {  // a word range of one stream's payload
         int s;
         uint64_t w0, w1;  // words from the stream's start
@@ -817,16 +834,18 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     // finest streams', the largest, first)
     auto build_header = [&](size_t s) {
         const StreamDesc& d = sd[s];
-        append_stream_header(parts[s].hdr, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
-                             unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
-                             h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
-                             (int)d.C);
+        build_stream_header(parts[s], ctx->arena, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
+                            unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
+                            h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
+                            (int)d.C);
     };
-    ContainerWriter cw(h, parts, *ctx->pool);
+    ctx->arena.reset();
+    ContainerWriter cw(h, parts, *ctx->pool, ctx->arena);
     std::atomic<int> ev_err{0};
-    // a group's copy seen complete once: later frames of the group make no
-    // CUDA call (concurrent calls from the pool's threads serialize in the
-    // driver, and frames queued behind a finished copy waited on each other)
+    // One thread waits for a group's copy, the others for that thread (0: not
+    // waited for, 1: being waited for, 2: complete): concurrent calls from the
+    // pool's threads serialize in the driver, and an event that blocks its
+    // waiter wakes it 0.35 ms late.
     std::unique_ptr<std::atomic<int>[]> copied(new std::atomic<int>[ngroups]);
     for (size_t i = 0; i < ngroups; ++i) copied[i].store(0);
     // zstd groups: every stream header first (nothing to wait for), then
@@ -839,9 +858,15 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
             return 2 + (size_t)(layer / lpg);
         },
         [&](size_t g) {
-            if (g == 0 || copied[g - 1].load(std::memory_order_acquire)) return;
-            if (cudaEventSynchronize(ev.e[g - 1]) != cudaSuccess) ev_err = 1;
-            copied[g - 1].store(1, std::memory_order_release);
+            if (g == 0) return;
+            std::atomic<int>& c = copied[g - 1];
+            int none = 0;
+            if (c.compare_exchange_strong(none, 1)) {
+                if (cudaEventSynchronize(ev.e[g - 1]) != cudaSuccess) ev_err = 1;
+                c.store(2, std::memory_order_release);
+            } else {
+                while (c.load(std::memory_order_acquire) != 2) std::this_thread::yield();
+            }
         },
         build_header);
     if (ev_err) {  // reports the device error
@@ -940,7 +965,8 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
     const int nstreams = 7 * kmax;
     p.kmax = kmax;
     p.sd.assign(nstreams, StreamDesc{});
-    p.hdr.assign(nstreams, StreamHeader{});
+    p.hdr.resize(nstreams);
+    ctx->arena.reset();
     p.unpred_prefix.assign(nstreams, {});
     std::atomic<int> bad{0};
     std::vector<const char*> why(nstreams, nullptr);
@@ -950,10 +976,10 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         const int k = (int)i / 7 + 1, b = (int)i % 7;
         const LevelDir& L = ps.lv[k];
         const StreamDir& d = L.s[b];
-        std::vector<uint8_t> raw(d.hdr_raw);
+        ArenaBlock raw;
         const int nch = (L.dx / L.C) * (L.dy / L.C) * (L.dz / L.C);
-        if (!decode_frame(bytes + d.data_off, d.hdr_stored, d.hdr_raw, raw.data())) bad = 1;
-        else if (!parse_stream_header(raw.data(), raw.size(), nch, L.C, elem, ps.version, p.hdr[i])) bad = 2;
+        if (!raw.take(ctx->arena, d.hdr_raw) || !decode_frame(bytes + d.data_off, d.hdr_stored, d.hdr_raw, raw.p)) bad = 1;
+        else if (!parse_stream_header(raw.p, d.hdr_raw, nch, L.C, elem, ps.version, p.hdr[i])) bad = 2;
         else why[i] = check_stream(h, L, d, p.hdr[i], p.unpred_prefix[i]);
     });
     if (bad) STZ_FAIL(STZ_ERR_FORMAT, bad == 1 ? "stream header frame does not decode" : "bad stream header");
@@ -1010,9 +1036,9 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         const StreamDesc& d = p.sd[i];
         std::memcpy(hs + o_sym + 2 * (size_t)d.cb_off, H.sym.data(), 2 * H.sym.size());
         std::memcpy(hs + o_len + d.cb_off, H.len.data(), H.len.size());
-        std::memcpy(hs + o_sub + 4 * d.sub_base, H.sub_off.data(), 4 * H.sub_off.size());
-        std::memcpy(hs + o_ch + 8 * d.chunk_base, H.chunk_word_off.data(), 8 * H.chunk_word_off.size());
-        if (H.n_unpred) std::memcpy(hs + o_ul + p.ulist_off[i] * elem, H.unpred.data(), H.unpred.size());
+        stream_copy(hs + o_sub + 4 * d.sub_base, H.sub_off.data(), 4 * H.sub_off.size());
+        stream_copy(hs + o_ch + 8 * d.chunk_base, H.chunk_word_off.data(), 8 * H.chunk_word_off.size());
+        if (H.n_unpred) stream_copy(hs + o_ul + p.ulist_off[i] * elem, H.unpred.data(), H.unpred.size());
     });
     lap.mark("layout + tables");
     // payload frames straight into the staging buffer
@@ -1105,7 +1131,8 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         }
         ctx->pool->parallel_for(bjobs.size(), [&](size_t i) {
             const Job& J = jobs[bjobs[i]];
-            if (!decode_frame(J.src, J.stored, J.raw, J.dst)) bad = 3;
+            if (J.stored == J.raw) stream_copy(J.dst, J.src, J.raw);
+            else if (!decode_frame(J.src, J.stored, J.raw, J.dst)) bad = 3;
         });
         if (bad) {
             sync_both();

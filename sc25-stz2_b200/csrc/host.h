@@ -1,6 +1,7 @@
 // Host-side pieces of the STZ B200 library: canonical Huffman codebooks, the
 // stream container, the ROI planner and a small thread pool for zstd.
 #pragma once
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <condition_variable>
@@ -9,6 +10,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -22,7 +24,9 @@ namespace stz {
 // pass over fresh pages).
 // Large byte blocks come from a small process-wide pool of recently freed
 // blocks (their pages stay mapped, so writing a new container does not fault
-// and zero fresh pages); the pool keeps at most 4 blocks and 2 GiB.
+// and zero fresh pages); the pool keeps at most 4 blocks and 2 GiB. Blocks are
+// rounded up by at most an eighth, so that the next stream of about the same
+// size fits a freed one, and large ones ask for huge pages.
 void* pooled_alloc(size_t bytes);
 void pooled_free(void* p, size_t bytes);
 
@@ -57,6 +61,54 @@ struct DefaultInitAlloc : std::allocator<T> {
 };
 using Bytes = std::vector<uint8_t, DefaultInitAlloc<uint8_t>>;
 
+// Host scratch of one context, handed out by the pool's threads during a call
+// and kept for the next: buffers of a call's frames cost more in page faults
+// and unmapping than the work on them does. reset() (no block in use) grows
+// it to what the calls since the last one asked for, up to kMax; take()
+// returns null when it is full, and the caller allocates for itself.
+class HostArena {
+public:
+    HostArena() = default;
+    HostArena(const HostArena&) = delete;
+    HostArena& operator=(const HostArena&) = delete;
+    ~HostArena() { pooled_free(p_, cap_); }
+    void reset()
+    {
+        const size_t want = std::min(used_.exchange(0), kMax);
+        if (want <= cap_) return;
+        pooled_free(p_, cap_);
+        p_ = static_cast<uint8_t*>(pooled_alloc(want));
+        cap_ = p_ ? want : 0;
+    }
+    uint8_t* take(size_t n)
+    {
+        if (n > kMax) return nullptr;
+        n = (n + 63) & ~(size_t)63;
+        const size_t at = used_.fetch_add(n);
+        return at + n <= cap_ ? p_ + at : nullptr;
+    }
+
+private:
+    static constexpr size_t kMax = (size_t)1 << 30;
+    uint8_t* p_ = nullptr;
+    size_t cap_ = 0;
+    std::atomic<size_t> used_{0};
+};
+
+// A block of an arena, or one of its own when the arena is full; null when
+// there is no memory.
+struct ArenaBlock {
+    uint8_t* p = nullptr;
+    std::unique_ptr<uint8_t[]> own;
+    uint8_t* take(HostArena& a, size_t n)
+    {
+        own.reset();
+        p = a.take(n);
+        if (!p) own.reset(p = new (std::nothrow) uint8_t[n]);
+        return p;
+    }
+};
+
 // ---- thread pool ----------------------------------------------------------
 class ThreadPool {
 public:
@@ -75,6 +127,13 @@ private:
     size_t n_ = 0, next_ = 0, active_ = 0;
     bool stop_ = false;
 };
+
+// memcpy for bulk data the copying core does not read again: the destination
+// is written past the caches.
+void stream_copy(void* dst, const void* src, size_t n);
+// Takes the lines of a buffer that cores have read out of their caches, so
+// that the next DMA write to it need not (nothing where the CPU cannot).
+void flush_lines(const void* p, size_t n);
 
 // ---- codebook -------------------------------------------------------------
 // Codebook of the container format for one histogram: symbols with a nonzero
@@ -156,16 +215,18 @@ bool parse_stream_header(const uint8_t* raw, size_t n, int nchunks, int C, size_
 
 // Writer input for one residual stream.
 struct StreamParts {
-    std::vector<uint8_t> hdr;        // raw stream header bytes
+    ArenaBlock hdr;                  // raw stream header bytes
+    size_t hdr_n = 0;
     const uint32_t* words = nullptr; // payload
     const uint64_t* chunk_word_off = nullptr;
     int layers = 0, chunks_per_layer = 0;
 };
 
-void append_stream_header(std::vector<uint8_t>& out, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
-                          uint32_t run_base, uint32_t run_n, uint64_t n_unpred, const void* unpred, size_t elem,
-                          const uint32_t* unpred_count, const uint64_t* chunk_word_off, const uint32_t* sub_off,
-                          int nchunks, int C);
+// The stream's header bytes into p.hdr, p.hdr_n.
+void build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
+                         uint32_t run_base, uint32_t run_n, uint64_t n_unpred, const void* unpred, size_t elem,
+                         const uint32_t* unpred_count, const uint64_t* chunk_word_off, const uint32_t* sub_off,
+                         int nchunks, int C);
 
 // A payload frame longer than this many bytes is zstd-compressed only when
 // zstd shrinks its first kZstdProbeBytes (stream headers and shorter frames
@@ -176,44 +237,40 @@ constexpr size_t kZstdProbeBytes = 4096;
 // frame per chunk z-layer of payload), zstd of the frames of a range of
 // streams on the pool (as soon as their bytes are on the host), then the
 // directory, the coarsest grid and every frame. `parts` stays alive and
-// unchanged until finish.
+// unchanged until finish, and the arena's blocks until the writer is gone.
 class ContainerWriter {
 public:
-    ContainerWriter(const FileHeader& h, std::vector<StreamParts>& parts, ThreadPool& pool);
-    void compress_streams(size_t s0, size_t s1);
+    ContainerWriter(const FileHeader& h, std::vector<StreamParts>& parts, ThreadPool& pool, HostArena& arena);
     // The frames in group order on the pool: group_of_frame(stream, layer)
     // (layer -1: the stream's header frame) gives a frame's group in
     // [0, ngroups) (anything else: not compressed by this call); a thread
-    // calls wait_group(g) before each frame of group g. build_header (may be
-    // empty): the job of stream s's header frame first calls it to fill
-    // parts[s].hdr, so each header is built and compressed by one job.
+    // calls wait_group(g) before each frame of group g. build_header: the job
+    // of stream s's header frame first calls it to fill parts[s].hdr, so each
+    // header is built and compressed by one job.
     void compress_groups(size_t ngroups, const std::function<size_t(size_t, int)>& group_of_frame,
                          const std::function<void(size_t)>& wait_group,
-                         const std::function<void(size_t)>& build_header = nullptr);
+                         const std::function<void(size_t)>& build_header);
     Bytes finish(const void* coarsest, const std::vector<LevelDir>& levels);
 
 private:
     struct Frame {
-        const uint8_t* src;
-        size_t n;
+        const uint8_t* src = nullptr;
+        size_t n = 0;
         bool payload = false;  // a chunk z-layer of payload (else a stream header)
-        std::unique_ptr<uint8_t[]> out;
+        ArenaBlock out;
         size_t stored = 0;
         bool raw = true;
-        const uint8_t* bytes() const { return raw ? src : out.get(); }
+        const uint8_t* bytes() const { return raw ? src : out.p; }
     };
     FileHeader h_;
     std::vector<StreamParts>& parts_;
     ThreadPool& pool_;
+    HostArena& arena_;
     std::vector<Frame> frames_;
     std::vector<size_t> first_;  // first frame of each stream (+ end)
     std::atomic<int64_t> busy_ns_{0};
     int64_t wall_ns_ = 0;
 };
-
-// All stages at once.
-Bytes write_container(const FileHeader& h, const void* coarsest, const std::vector<LevelDir>& levels,
-                      std::vector<StreamParts>& parts, ThreadPool& pool);
 
 // ---- ROI planner (FD5:1578-1839) -------------------------------------------
 struct AxisRange {

@@ -128,6 +128,14 @@ struct Prepared {
     LearnedModel* d_models = nullptr;  // per level k (index k), when the stream has learned corrections
     void* d_tables = nullptr;          // decode tables per stream (launch_build_tables)
     bool base_valid = false;  // *base holds the decoded base grid (level K-2 output) for box queries
+    std::vector<StreamHeader>* hdr_home = nullptr;  // where a one-off decode's headers go back to (their memory is kept)
+    Prepared() = default;
+    Prepared(const Prepared&) = delete;
+    Prepared& operator=(const Prepared&) = delete;
+    ~Prepared()
+    {
+        if (hdr_home) hdr_home->swap(hdr);
+    }
 };
 
 // Where the level kernels evaluate the learned network: block-wide on the
@@ -258,11 +266,18 @@ struct stz_context {
         stream_words, payload, sd, work, ids, uwork, ulist, books, cb_scratch, minmax, packed, rbits, out, mid, boxes,
         tiles, models, eval, rstats, staged_full;
     stz::PinBuf h_hist, h_meta, h_meta2, h_payload, h_stage, h_io, h_small;
+    size_t io_read = 0, payload_read = 0;  // bytes of h_io and h_payload that the host read in the last compress
     stz::PinBuf h_xfer[2];  // staging chunks of host <-> device copies of pageable caller buffers
     // device buffers lent to one-off decodes
     stz::DevBuf p_stage, p_coarsest, p_base;
+    // host memory kept between calls: frames and headers of a call, and the
+    // parsed headers of one-off decodes
+    stz::HostArena arena;
+    std::vector<stz::StreamHeader> hdr_scratch;
     void borrow(stz::Prepared& p)
     {
+        p.hdr.swap(hdr_scratch);
+        p.hdr_home = &hdr_scratch;
         p.stage = &p_stage;
         p.coarsest = &p_coarsest;
         p.base = &p_base;
