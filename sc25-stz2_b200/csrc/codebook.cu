@@ -13,8 +13,12 @@
 // outside the window), and a codebook of tens of thousands of symbols took
 // milliseconds of sorting and merging. Measured from the histograms to the
 // code tables (one B200, 16 host cores), host before and both kernels here
-// now: 64^3 f32 0.52 -> 0.058 ms, 512^3 f32 at rel 1e-3 0.25 -> 0.085 ms and
-// at 1e-4 1.4 -> 0.11 ms, 384x384x256 f64 fronts at 1e-6 12-14 -> 1.07 ms.
+// now: 64^3 f32 0.52 -> 0.058 ms, 512^3 f32 at rel 1e-3 0.25 -> 0.073 ms and
+// at 1e-4 1.4 -> 0.11 ms, 384x384x256 f64 fronts at 1e-6 (codebooks of up to
+// 60 K symbols) 12-14 -> 0.69 ms, 1.07 ms of it before the searches of a
+// thread ran four side by side and the sort loaded four items ahead. The
+// merges of up to kSmallBook symbols are one warp's work in shared memory:
+// 0.085 -> 0.073 ms on the 512^3 field at 1e-3.
 //
 // The merging is sequential in the textbook form, but every weight not above
 // the sum t of the two smallest is consumed before the first merge of that
@@ -36,6 +40,7 @@ namespace {
 
 constexpr int kCbThreads = 1024;
 constexpr int kCbWarps = kCbThreads / 32;
+constexpr uint32_t kSmallBook = 512;  // symbols whose merges one warp makes (14 KB of lists)
 constexpr int kMaxRounds = 192;  // rounds <= 2 log2(total count) + 2
 constexpr int kMaxDepth = 80;    // depth <= 1.45 log2(total count) + 2
 
@@ -99,12 +104,14 @@ __device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* wsum, uin
     return (w ? wsum[w - 1] : 0u) + incl - v;
 }
 
-// Stable counting sort of n items by an 8-bit digit: put(i, pos) for item i
-// at its place. Every warp owns n / 32 consecutive items and a row of 256
+// Stable counting sort of n items by an 8-bit digit: put(i, key, pos) for item
+// i at its place. Every warp owns n / 32 consecutive items and a row of 256
 // counters, so a pass has no barrier between its counting and its ranking
-// steps. cnt: kCbWarps x 256 words of shared memory.
-template <class Digit, class Put>
-__device__ __forceinline__ void counting_pass(uint32_t n, uint32_t* cnt, uint32_t* wsum, Digit&& digit, Put&& put)
+// steps; four items per lane are loaded ahead of both. cnt: kCbWarps x 256
+// words of shared memory.
+template <class Key, class Load, class Digit, class Put>
+__device__ __forceinline__ void counting_pass(uint32_t n, uint32_t* cnt, uint32_t* wsum, Load&& load, Digit&& digit,
+                                              Put&& put)
 {
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t per = ((n + kCbThreads - 1) / kCbThreads) * 32;
@@ -112,12 +119,20 @@ __device__ __forceinline__ void counting_pass(uint32_t n, uint32_t* cnt, uint32_
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kCbWarps * 256; i += kCbThreads) cnt[i] = 0;
     __syncthreads();
-    for (uint32_t i0 = a; i0 < b; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const uint32_t d = i < b ? digit(i) : 256u;
-        const uint32_t same = __match_any_sync(0xffffffffu, d);
-        if (i < b && (uint32_t)(__ffs(same) - 1) == lane) cnt[w * 256 + d] += __popc(same);
-        __syncwarp();
+    for (uint32_t i0 = a; i0 < b; i0 += 128) {
+        Key key[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i0 + 32 * j + lane < b) key[j] = load(i0 + 32 * j + lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (i0 + 32 * j >= b) break;  // uniform per warp
+            const bool in = i0 + 32 * j + lane < b;
+            const uint32_t d = in ? digit(key[j]) : 256u;
+            const uint32_t same = __match_any_sync(0xffffffffu, d);
+            if (in && (uint32_t)(__ffs(same) - 1) == lane) cnt[w * 256 + d] += __popc(same);
+            __syncwarp();
+        }
     }
     __syncthreads();
     // counters -> first places, digit by digit and warp by warp within one:
@@ -136,20 +151,132 @@ __device__ __forceinline__ void counting_pass(uint32_t n, uint32_t* cnt, uint32_
         }
     }
     __syncthreads();
-    for (uint32_t i0 = a; i0 < b; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const uint32_t d = i < b ? digit(i) : 256u;
-        const uint32_t same = __match_any_sync(0xffffffffu, d);
-        uint32_t first = 0;
-        if (i < b) first = cnt[w * 256 + d];
-        __syncwarp();
-        if (i < b) {
-            if ((uint32_t)(__ffs(same) - 1) == lane) cnt[w * 256 + d] = first + __popc(same);
-            put(i, first + __popc(same & ((1u << lane) - 1u)));
+    for (uint32_t i0 = a; i0 < b; i0 += 128) {
+        Key key[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i0 + 32 * j + lane < b) key[j] = load(i0 + 32 * j + lane);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (i0 + 32 * j >= b) break;  // uniform per warp
+            const uint32_t i = i0 + 32 * j + lane;
+            const bool in = i < b;
+            const uint32_t d = in ? digit(key[j]) : 256u;
+            const uint32_t same = __match_any_sync(0xffffffffu, d);
+            uint32_t first = 0;
+            if (in) first = cnt[w * 256 + d];
+            __syncwarp();
+            if (in) {
+                if ((uint32_t)(__ffs(same) - 1) == lane) cnt[w * 256 + d] = first + __popc(same);
+                put(i, key[j], first + __popc(same & ((1u << lane) - 1u)));
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
     __syncthreads();
+}
+
+// The threads that merge one codebook: the CTA, or one warp for a small one,
+// whose rounds cost the latency of their barriers.
+struct WholeCta {
+    static constexpr uint32_t size = kCbThreads;
+    static __device__ __forceinline__ uint32_t id() { return threadIdx.x; }
+    static __device__ __forceinline__ void sync() { __syncthreads(); }
+    static __device__ __forceinline__ uint32_t count(bool p) { return (uint32_t)__syncthreads_count(p); }
+};
+struct OneWarp {
+    static constexpr uint32_t size = 32;
+    static __device__ __forceinline__ uint32_t id() { return threadIdx.x & 31; }
+    static __device__ __forceinline__ void sync() { __syncwarp(); }
+    static __device__ __forceinline__ uint32_t count(bool p) { return __popc(__ballot_sync(0xffffffffu, p)); }
+};
+
+// For items k < n: the number of the sorted list's first m entries that come
+// before value(k), to done(k, value, rank). Up to four searches per thread
+// side by side: the lists of a large codebook lie in L2, and a search is a
+// chain of its latency.
+template <class Group, class Value, class Before, class Done>
+__device__ __forceinline__ void ranks(uint32_t n, uint32_t m, Value&& value, Before&& before, Done&& done)
+{
+    const uint32_t top = m ? 1u << (31 - __clz(m)) : 0u;
+    uint32_t k0 = Group::id();
+    if (Group::size == kCbThreads)
+        for (; k0 + kCbThreads < n; k0 += 4 * kCbThreads) {
+            uint64_t v[4];
+            uint32_t pos[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (k0 + j * kCbThreads < n) v[j] = value(k0 + j * kCbThreads);
+            for (uint32_t step = top; step; step >>= 1)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (k0 + j * kCbThreads < n && pos[j] + step <= m && before(pos[j] + step - 1, v[j])) pos[j] += step;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (k0 + j * kCbThreads < n) done(k0 + j * kCbThreads, v[j], pos[j]);
+        }
+    for (; k0 < n; k0 += Group::size) {
+        const uint64_t v = value(k0);
+        uint32_t pos = 0;
+        for (uint32_t step = top; step; step >>= 1)
+            if (pos + step <= m && before(pos + step - 1, v)) pos += step;
+        done(k0, v, pos);
+    }
+}
+
+// All merges of n sorted symbols: weights to node, parents to up, the first
+// merge of every round to first; returns the rounds, and the merges in m.
+template <class Group>
+__device__ __forceinline__ uint32_t merge_rounds(uint32_t n, const uint64_t* leaf, uint64_t* node, uint64_t* merged,
+                                                 uint32_t* up, uint32_t* first, uint32_t& m)
+{
+    const uint32_t id = Group::id();
+    uint32_t i = 0, j = 0, rounds = 0;  // first unmerged symbol, first unmerged merge
+    m = 0;
+    if (id == 0) first[0] = 0;
+    while (n - i + (m - j) > 1) {
+        const uint64_t none = ~0ull;
+        const uint64_t l0 = i < n ? leaf[i] >> 32 : none, l1 = i + 1 < n ? leaf[i + 1] >> 32 : none;
+        const uint64_t q0 = j < m ? node[j] : none, q1 = j + 1 < m ? node[j + 1] : none;
+        // sum of the two smallest
+        const uint64_t t = l0 <= q0 ? l0 + min(l1, q0) : q0 + min(l0, q1);
+        // symbols and merges of weight <= t
+        uint32_t a = 0, b = 0;
+        for (;;) {
+            const uint32_t k = i + a + id, c = Group::count(k < n && (leaf[k] >> 32) <= t);
+            a += c;
+            if (c < Group::size) break;
+        }
+        for (;;) {
+            const uint32_t k = j + b + id, c = Group::count(k < m && node[k] <= t);
+            b += c;
+            if (c < Group::size) break;
+        }
+        if ((a + b) & 1) {  // the last of them waits for the next round (on equal weights the merge is last)
+            if (b && (a == 0 || node[j + b - 1] >= (leaf[i + a - 1] >> 32))) --b;
+            else --a;
+        }
+        // places in merged order (on equal weights the symbol is first); a
+        // merge's pair is its parent
+        ranks<Group>(a, b, [&](uint32_t k) { return leaf[i + k] >> 32; },
+                     [&](uint32_t x, uint64_t w) { return node[j + x] < w; },
+                     [&](uint32_t k, uint64_t w, uint32_t r) { merged[k + r] = w; });
+        ranks<Group>(b, a, [&](uint32_t k) { return node[j + k]; },
+                     [&](uint32_t x, uint64_t w) { return (leaf[i + x] >> 32) <= w; },
+                     [&](uint32_t k, uint64_t w, uint32_t r) {
+                         merged[k + r] = w;
+                         up[j + k] = m + ((k + r) >> 1);
+                     });
+        Group::sync();
+        const uint32_t pairs = (a + b) >> 1;
+        for (uint32_t k = id; k < pairs; k += Group::size) node[m + k] = merged[2 * k] + merged[2 * k + 1];
+        i += a, j += b, m += pairs;
+        ++rounds;
+        if (id == 0) first[rounds] = m;
+        Group::sync();
+        if (rounds == kMaxRounds) break;  // not reached: the smallest weight doubles every two rounds
+    }
+    return rounds;
 }
 
 // Code lengths of both codebooks of every stream: blockIdx.x the stream,
@@ -161,7 +288,8 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook(const StreamDesc* __res
                                                          const uint64_t* __restrict__ scratch_off, uint8_t* scratch,
                                                          BookRecord* __restrict__ rec)
 {
-    __shared__ uint32_t cnt[kCbWarps * 256];  // the sort's counters; before it, the bitmap of used codes
+    // the sort's counters; before it, the bitmap of used codes; after it, the lists of a small codebook
+    __shared__ __align__(8) uint32_t cnt[kCbWarps * 256];
     __shared__ uint32_t wsum[kCbWarps];
     __shared__ uint32_t first[kMaxRounds + 1];  // first merge of every round
     __shared__ uint32_t icnt[kMaxDepth];
@@ -190,9 +318,18 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook(const StreamDesc* __res
         c0 = R > (uint32_t)kHistWindow / 2 ? R - kHistWindow / 2 : 0u;
         c1 = min(R2, R + kHistWindow / 2);
     }
-    for (uint32_t c = (c0 & ~31u) + tid; c < ((c1 + 31) & ~31u); c += kCbThreads) {
-        const uint32_t m = __ballot_sync(0xffffffffu, c >= c0 && c < c1 && h[c] != 0);
-        if (lane == 0) used[c >> 5] = m;
+    for (uint32_t c = (c0 & ~31u) + tid; c < ((c1 + 31) & ~31u); c += 8 * kCbThreads) {
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t x = c + j * kCbThreads;
+            v[j] = x >= c0 && x < c1 ? h[x] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t x = c + j * kCbThreads, m = __ballot_sync(0xffffffffu, v[j] != 0);
+            if (lane == 0 && m) used[x >> 5] = m;
+        }
     }
     __syncthreads();
     uint32_t run_base = 0;
@@ -281,73 +418,29 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook(const StreamDesc* __res
     for (uint32_t sh = 32; sh < 64 && (maxw >> (sh - 32)); sh += 8) {
         const uint64_t* src = B.key[cur];
         uint64_t* dst = B.key[cur ^ 1];
-        counting_pass(
-            n, cnt, wsum, [&](uint32_t i) { return (uint32_t)(src[i] >> sh) & 255u; },
-            [&](uint32_t i, uint32_t p) { dst[p] = src[i]; });
+        counting_pass<uint64_t>(
+            n, cnt, wsum, [&](uint32_t i) { return src[i]; },
+            [&](uint64_t k) { return (uint32_t)(k >> sh) & 255u; },
+            [&](uint32_t, uint64_t k, uint32_t p) { dst[p] = k; });
         cur ^= 1;
     }
     const uint64_t* leaf = B.key[cur];
-    uint64_t* merged = B.key[cur ^ 1];
-    uint64_t* node = B.node;
     uint32_t* up = B.up;
-
-    // ---- rounds of merges ----
-    uint32_t i = 0, j = 0, m = 0, rounds = 0;  // first unmerged symbol, first unmerged merge, merges made
-    if (tid == 0) first[0] = 0;
-    while (n - i + (m - j) > 1) {
-        const uint64_t none = ~0ull;
-        const uint64_t l0 = i < n ? leaf[i] >> 32 : none, l1 = i + 1 < n ? leaf[i + 1] >> 32 : none;
-        const uint64_t q0 = j < m ? node[j] : none, q1 = j + 1 < m ? node[j + 1] : none;
-        // sum of the two smallest
-        const uint64_t t = l0 <= q0 ? l0 + min(l1, q0) : q0 + min(l0, q1);
-        // symbols and merges of weight <= t
-        uint32_t a = 0, b = 0;
-        for (;;) {
-            const uint32_t k = i + a + tid;
-            const uint32_t c = __syncthreads_count(k < n && (leaf[k] >> 32) <= t);
-            a += c;
-            if (c < kCbThreads) break;
-        }
-        for (;;) {
-            const uint32_t k = j + b + tid;
-            const uint32_t c = __syncthreads_count(k < m && node[k] <= t);
-            b += c;
-            if (c < kCbThreads) break;
-        }
-        if ((a + b) & 1) {  // the last of them waits for the next round (on equal weights the merge is last)
-            if (b && (a == 0 || node[j + b - 1] >= (leaf[i + a - 1] >> 32))) --b;
-            else --a;
-        }
-        // places in merged order; a merge's pair is its parent
-        for (uint32_t k = tid; k < a; k += kCbThreads) {
-            const uint64_t w = leaf[i + k] >> 32;
-            uint32_t lo = 0, hi = b;  // merges lighter than w
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (node[j + mid] < w) lo = mid + 1;
-                else hi = mid;
-            }
-            merged[k + lo] = w;
-        }
-        for (uint32_t k = tid; k < b; k += kCbThreads) {
-            const uint64_t w = node[j + k];
-            uint32_t lo = 0, hi = a;  // symbols not heavier than w
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if ((leaf[i + mid] >> 32) <= w) lo = mid + 1;
-                else hi = mid;
-            }
-            merged[k + lo] = w;
-            up[j + k] = m + ((k + lo) >> 1);
+    uint32_t m, rounds;
+    if (n <= kSmallBook) {  // in shared memory, where the sort's counters were
+        uint64_t* sl = reinterpret_cast<uint64_t*>(cnt);
+        for (uint32_t k = tid; k < n; k += kCbThreads) sl[k] = leaf[k];
+        leaf = sl;
+        up = reinterpret_cast<uint32_t*>(sl + 3 * kSmallBook);
+        __syncthreads();
+        if (tid < 32) {
+            rounds = merge_rounds<OneWarp>(n, leaf, sl + kSmallBook, sl + 2 * kSmallBook, up, first, m);
+            if (tid == 0) wsum[0] = rounds, wsum[1] = m;
         }
         __syncthreads();
-        const uint32_t pairs = (a + b) >> 1;
-        for (uint32_t k = tid; k < pairs; k += kCbThreads) node[m + k] = merged[2 * k] + merged[2 * k + 1];
-        i += a, j += b, m += pairs;
-        ++rounds;
-        if (tid == 0) first[rounds] = m;
-        __syncthreads();
-        if (rounds == kMaxRounds) break;  // not reached: the smallest weight doubles every two rounds
+        rounds = wsum[0], m = wsum[1];
+    } else {
+        rounds = merge_rounds<WholeCta>(n, leaf, B.node, B.key[cur ^ 1], up, first, m);
     }
 
     // ---- depths of the merges, last round first; merges of each depth ----
@@ -356,18 +449,38 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook(const StreamDesc* __res
     __syncthreads();
     for (uint32_t r = rounds; r-- > 0;) {
         const uint32_t x1 = first[r + 1];
-        for (uint32_t x0 = first[r]; x0 < x1; x0 += kCbThreads) {
+        uint32_t x0 = first[r];
+        for (; x0 + kCbThreads < x1; x0 += 4 * kCbThreads) {
+            uint32_t d[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t x = x0 + q * kCbThreads + tid;
+                d[q] = x < x1 && x != m - 1 ? up[x] : m - 1;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t x = x0 + q * kCbThreads + tid;
+                d[q] = x < x1 ? (x == m - 1 ? 0u : min(up[d[q]] + 1u, (uint32_t)kMaxDepth - 1)) : (uint32_t)kMaxDepth;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t x = x0 + q * kCbThreads + tid;
+                const uint32_t same = __match_any_sync(0xffffffffu, d[q]);
+                if (x < x1) {
+                    if ((uint32_t)(__ffs(same) - 1) == lane) atomicAdd(&icnt[d[q]], __popc(same));
+                    up[x] = d[q];
+                }
+            }
+        }
+        for (; x0 < x1; x0 += kCbThreads) {
             const uint32_t x = x0 + tid;
             uint32_t d = kMaxDepth;
-            if (x < x1) {
-                d = x == m - 1 ? 0u : min(up[up[x]] + 1u, (uint32_t)kMaxDepth - 1);
-            }
+            if (x < x1) d = x == m - 1 ? 0u : min(up[up[x]] + 1u, (uint32_t)kMaxDepth - 1);
             const uint32_t same = __match_any_sync(0xffffffffu, d);
             if (x < x1) {
                 if ((uint32_t)(__ffs(same) - 1) == lane) atomicAdd(&icnt[d], __popc(same));
+                up[x] = d;
             }
-            __syncwarp();
-            if (x < x1) up[x] = d;
         }
         __syncthreads();
     }
@@ -408,8 +521,8 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook(const StreamDesc* __res
     }
     __syncthreads();
     unsigned long long bits = 0;
+    uint32_t l = kMaxCodeLen;  // lengths fall along the list
     for (uint32_t k = tid; k < n; k += kCbThreads) {
-        uint32_t l = kMaxCodeLen;
         while (l > 0 && k >= lpos[l] + lcnt[l]) --l;
         const uint64_t e = leaf[k];
         B.len[(uint32_t)e] = (uint8_t)l;
@@ -462,11 +575,12 @@ __global__ void __launch_bounds__(kCbThreads) k_codebook_emit(StreamDesc* sd,
         info[blockIdx.x] = {off, r.n, d.run_base, d.run_n};
     }
     uint32_t* tab = ctab + (size_t)blockIdx.x * 2 * R;
-    counting_pass(
-        r.n, cnt, wsum, [&](uint32_t i) { return (uint32_t)B.len[i]; },
-        [&](uint32_t i, uint32_t p) {
-            const uint32_t l = B.len[i];
-            const uint16_t sym = B.sym[i];
+    counting_pass<uint32_t>(
+        r.n, cnt, wsum, [&](uint32_t i) { return (uint32_t)B.len[i] << 16 | B.sym[i]; },
+        [&](uint32_t k) { return k >> 16; },
+        [&](uint32_t, uint32_t k, uint32_t p) {
+            const uint32_t l = k >> 16;
+            const uint16_t sym = (uint16_t)k;
             cb_sym[off + p] = sym;
             cb_len[off + p] = (uint8_t)l;
             tab[sym] = l ? (first_code[l] + (p - first_idx[l])) << 5 | l : 0u;

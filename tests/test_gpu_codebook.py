@@ -2,7 +2,8 @@
 fields whose finest-level code histograms are chosen. With a zero coarse grid
 every prediction is zero, so at multipliers 1 and eb 0.5 a fine value k is
 coded as radius + k. The cases sit where the construction can go wrong: one
-and two symbols, all-equal counts (ties), Fibonacci counts (the longest codes,
+and two symbols, all-equal counts (ties), symbol counts around the one-warp
+and whole-CTA merges, Fibonacci counts (the longest codes,
 past the 24-bit cap), geometric counts, codes over the whole range with
 unpredictable values, a radius that leaves no room for run symbols, and
 planes of one code (no run symbols at all)."""
@@ -25,6 +26,9 @@ def _codes(kind, n, rng):
         return rng.integers(0, 2, n)
     if kind == "equal":
         return np.arange(n) % 4096 - 2048
+    if kind.startswith("first"):  # that many codes, some of equal counts
+        k = int(kind[5:])
+        return np.arange(n) % k * (1 + np.arange(n) % 3 % 2) % k - k // 2
     if kind == "wide":
         return np.arange(n) % 40000 - 20000
     if kind == "fibonacci":
@@ -47,6 +51,10 @@ def _codes(kind, n, rng):
     ("one", (64, 64, 64), 32768, 32),
     ("two", (64, 64, 64), 32768, 32),
     ("equal", (64, 128, 64), 32768, 32),
+    ("first511", (64, 64, 64), 32768, 32),
+    ("first512", (64, 64, 64), 32768, 32),
+    ("first513", (64, 64, 64), 32768, 32),
+    ("first1025", (64, 64, 64), 32768, 32),
     ("wide", (128, 128, 128), 32768, 32),
     ("fibonacci", (128, 128, 192), 32768, 32),
     ("geometric", (128, 64, 64), 32768, 32),
