@@ -187,6 +187,17 @@ template <typename T>
 stz_status level_error_bounds(stz_context* ctx, const T* field, size_t N, const stz_opts& o, int K, double& eb,
                               std::vector<double>& ebk);
 
+// No chunk of the listed unpredictable values is larger than
+// unpred_little_codes().
+inline bool unpred_little(const std::vector<StreamDesc>& sd, const UnpredWork* w, size_t n)
+{
+    for (size_t i = 0; i < n; ++i) {
+        const uint32_t C = sd[w[i].stream].C;
+        if (C * C * C > unpred_little_codes()) return false;
+    }
+    return true;
+}
+
 // CTA work items for chunk lists: groups of up to kCoderThreads / C chunks.
 void add_work(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint32_t stream, const uint32_t* chunks,
               size_t n, int C);

@@ -28,7 +28,7 @@ def _codes(kind, n, rng):
         return np.arange(n) % 4096 - 2048
     if kind.startswith("first"):  # that many codes, some of equal counts
         k = int(kind[5:])
-        return np.arange(n) % k * (1 + np.arange(n) % 3 % 2) % k - k // 2
+        return np.arange(n) % k - k // 2
     if kind == "wide":
         return np.arange(n) % 40000 - 20000
     if kind == "fibonacci":
