@@ -677,7 +677,10 @@ __global__ void __launch_bounds__(kLaneThreads) k_encode(const CtaWork* __restri
 //   * One lookup gives the length of any code but the few whose table prefix
 //     spans two lengths: canonical codes of one length are one interval. A
 //     code of up to kLutBits bits also gets its symbol or run length, a
-//     longer one its canonical index.
+//     longer one its canonical index. For those few the entry says where the
+//     search through the lengths starts, which then ends within a step or two.
+//   * The counting passes, two thirds of the steps, take only the length and
+//     the run length from the entry.
 //   * The symbols of longer codes are looked up when the plane is stored,
 //     many at a time, so no lane waits for one in the middle of its chain.
 //     Where long codes are common (DecodeTables::by_index) the plane holds
@@ -685,20 +688,26 @@ __global__ void __launch_bounds__(kLaneThreads) k_encode(const CtaWork* __restri
 // Before, table, payload words and symbols were read through L1 in the chain,
 // the length of a long code was searched there, and dense streams of large
 // launches had one thread per plane, whose lanes diverged. Launch times on one
-// B200, before and now (levels below the finest, then its two halves):
-//   512^3 f32 at 1e-3          0.139 / 0.160 / 0.131 -> 0.127 / 0.166 / 0.126 ms
-//   512^3 f32 at 1e-4          0.221 / 1.036 / 0.711 -> 0.198 / 0.496 / 0.315 ms
-//   384x384x256 f64 at 1e-6    0.230 / 0.560 / 0.520 -> 0.079 / 0.270 / 0.229 ms
-//   its boxes of 16-128 a side 0.156 -> 0.068 ms a box
+// B200, then and now (levels below the finest and its two halves together):
+//   512^3 f32 at 1e-3          0.430 -> 0.338 ms
+//   512^3 f32 at 1e-4          1.968 -> 0.687 ms
+//   384x384x256 f64 at 1e-6    1.310 -> 0.464 ms
+//   its boxes of 16-128 a side 0.156 -> 0.048 ms a box
+// (With one step function for counting and placing, the search from kLutBits
+// up and through L1, and one build for launches of all sizes: 0.41, 0.86, 0.56
+// and 0.068 ms.)
 // Tried as well: one lane per plane in lockstep (windows of codes in shared
 // memory, payload rings filled by asynchronous copies), 0.17 / 0.62 / 0.42 ms
 // at 1e-4 and a chain of 1024 symbols in every small launch; several symbols
 // per lookup in the counting passes (fewer instructions, more table to load:
 // even); four lanes' worth of planes per warp for all streams (fewer warps
-// resident: slower).
+// resident: slower); only the planes that a box needs, as work items of equal
+// plane ranges (a box's decode is the chain of two or three planes in each
+// warp, and chunks with unpredictable values start at plane 0: even).
 
 // lut entry: code length in bits 0-4 (0: the prefix spans lengths, holds long
-// run symbols, or no code); kLutRun: a run symbol, its run length in
+// run symbols, or no code; bits 16-31 then hold the shortest length above
+// kLutBits that a code under it may have); kLutRun: a run symbol, its run length in
 // bits 16-31; kLutLong: a longer code, its canonical index is its value plus
 // bits 16-31 (mod 2^16); else the symbol in bits 16-31 (its canonical index
 // where the stream decodes by index).
@@ -728,7 +737,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_build_tables(const StreamDesc
     __shared__ uint32_t cnt[kMaxCodeLen + 1], first_code[kMaxCodeLen + 1], first_idx[kMaxCodeLen + 1];
     __shared__ uint32_t start[kMaxCodeLen + 1];  // first index of each length (the list is in length order)
     __shared__ uint32_t rlo[kMaxCodeLen + 1], rcnt[kMaxCodeLen + 1], roff[kMaxCodeLen + 1];
-    __shared__ uint32_t by_index;
+    __shared__ uint32_t by_index, longest;
     const uint32_t tid = threadIdx.x;
     if (tid <= kMaxCodeLen) start[tid] = 0xffffffffu, rlo[tid] = 0xffffffffu, rcnt[tid] = 0;
     __syncthreads();
@@ -748,7 +757,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_build_tables(const StreamDesc
             cnt[l] = start[l] == 0xffffffffu ? 0u : (uint32_t)end - start[l];
             if (cnt[l]) end = (int)start[l];
         }
-        uint32_t code = 0, idx = cnt[0], ro = 0, longest = 0, mass = 0;
+        uint32_t code = 0, idx = cnt[0], ro = 0, mass = 0;
+        longest = 0;
         first_code[0] = first_idx[0] = roff[0] = 0;
         for (int l = 1; l <= kMaxCodeLen; ++l) {
             code = (code + (l > 1 ? cnt[l - 1] : 0)) << 1;
@@ -794,6 +804,11 @@ __global__ void __launch_bounds__(kBuildThreads) k_build_tables(const StreamDesc
                     e = l | kLutLong | b << 16;
             }
         }
+        if (!e) {  // as DecodeCtx::slow looks for the prefix's first code
+            uint32_t l = kLutBits + 1;
+            while (l <= longest && j << (kMaxCodeLen - kLutBits) >= (first_code[l] + cnt[l]) << (kMaxCodeLen - l)) ++l;
+            e = l << 16;
+        }
         t.lut[j] = e;
     }
 }
@@ -809,35 +824,59 @@ struct DecodeSmem {
     uint4 out[kDecodeWarps][kMaxPlane / 8];
     uint4 stage[kDecodeWarps][kStageWords / 4];
     uint32_t late[kDecodeWarps][kMaxPlane / 32];  // entries that hold the index of a long code
+    uint4 len[kMaxCodeLen + 1];                   // as DecodeTables
+    uint32_t max_len;
 };
 
 // Symbol decoding from a stream's tables, the lookup table itself in shared
 // or in global memory.
 struct DecodeCtx {
     const uint32_t* lut;
+    const uint4* len;  // where lut is
+    uint32_t longest;
     const DecodeTables* __restrict__ t;
+    template <bool SMEM>
+    __device__ __forceinline__ uint32_t entry(uint32_t bits) const
+    {
+        return SMEM ? lut[bits >> (32 - kLutBits)] : __ldg(lut + (bits >> (32 - kLutBits)));
+    }
     // The code at the top of bits: its length, and symbol or run length, or
     // canonical index (late).
     template <bool SMEM>
     __device__ __forceinline__ void symbol(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
     {
-        const uint32_t e = SMEM ? lut[bits >> (32 - kLutBits)] : __ldg(lut + (bits >> (32 - kLutBits)));
+        const uint32_t e = entry<SMEM>(bits);
         l = e & 31u, val = e >> 16, run = e & kLutRun, late = e & kLutLong;
         if (late) val = (bits >> (32 - l)) + val & 0xffffu;
-        if (l == 0) slow(bits, l, val, run, late);
+        if (l == 0) slow<SMEM>(bits, l, val, run, late);
     }
+    // Its length, and how many codes it stands for.
+    template <bool SMEM>
+    __device__ __forceinline__ void count(uint32_t bits, uint32_t& l, uint32_t& n) const
+    {
+        const uint32_t e = entry<SMEM>(bits);
+        l = e & 31u, n = e & kLutRun ? e >> 16 : 1u;
+        if (l == 0) {
+            uint32_t val = e >> 16;
+            bool run, late;
+            slow<SMEM>(bits, l, val, run, late);
+            n = run ? val : 1u;
+        }
+    }
+    // val: the length to start from.
+    template <bool SMEM>
     __device__ __forceinline__ void slow(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
     {
-        const uint32_t v = bits >> (32 - kMaxCodeLen), longest = __ldg(&t->max_len);
-        l = kLutBits + 1;
-        while (l <= longest && v >= __ldg(&t->len[l].x)) ++l;
+        const uint32_t v = bits >> (32 - kMaxCodeLen);
+        l = val;
+        while (l <= longest && v >= (SMEM ? len[l].x : __ldg(&len[l].x))) ++l;
         run = false, late = true;
         if (l > longest) {  // no code (corrupt stream): the codebook's first symbol, one bit
             l = 1;
             val = 0;
             return;
         }
-        const uint4 e = __ldg(&t->len[l]);
+        const uint4 e = SMEM ? len[l] : __ldg(&len[l]);
         const uint32_t i = (bits >> (32 - l)) + e.y, r = i - e.z;
         run = r < (e.w & 0xffffu);
         val = run ? __ldg(&t->run[(e.w >> 16) + r]) : i;
@@ -865,10 +904,9 @@ __device__ __forceinline__ void decode_plane(const DecodeCtx& dc, const Words& w
     auto count = [&]() {
         cnt = 0;
         while (end < stop) {
-            uint32_t l, val;
-            bool run, late;
-            dc.symbol<SMEM>(peek(w, end), l, val, run, late);
-            cnt += run ? val : 1u;
+            uint32_t l, n;
+            dc.count<SMEM>(peek(w, end), l, n);
+            cnt += n;
             end += l;
         }
     };
@@ -958,7 +996,7 @@ __device__ __forceinline__ void decode_direct(const StreamDesc& s, const DecodeT
     const uint16_t* __restrict__ syms = cb_sym + s.cb_off;
     const uint32_t fill = fill_code(s, syms);
     const bool by_index = t->by_index;
-    const DecodeCtx dc{t->lut, t};
+    const DecodeCtx dc{t->lut, t->len, t->max_len, t};
     for (uint32_t base = first * G; base < np; base += nwarps * G) {
         const bool active = base + gi < np;
         const PlaneAt a = plane_at(s, chunks, active ? base + gi : base, active, sub_off, chunk_word_off, payload, codes);
@@ -1008,7 +1046,7 @@ __device__ __forceinline__ void decode_buffered(DecodeSmem& sm, const StreamDesc
         late[all] = 0;
     }
     __syncwarp();
-    const DecodeCtx dc{sm.lut, t};
+    const DecodeCtx dc{sm.lut, sm.len, sm.max_len, t};
     for (uint32_t base = first * G; base < np; base += nwarps * G) {
         const bool active = base + gi < np;
         const PlaneAt a = plane_at(s, chunks, active ? base + gi : base, active, sub_off, chunk_word_off, payload, codes);
@@ -1089,6 +1127,8 @@ __device__ __forceinline__ void load_table(DecodeSmem& sm, const DecodeTables* _
     const uint4* __restrict__ src = reinterpret_cast<const uint4*>(t->lut);
     for (uint32_t i = threadIdx.x; i < (1u << kLutBits) / 4; i += kDecodeThreads)
         reinterpret_cast<uint4*>(sm.lut)[i] = __ldg(src + i);
+    if (threadIdx.x <= kMaxCodeLen) sm.len[threadIdx.x] = __ldg(t->len + threadIdx.x);
+    if (threadIdx.x == 0) sm.max_len = t->max_len;
     __syncthreads();
 }
 
@@ -1106,15 +1146,16 @@ __host__ __device__ inline uint32_t decode_slices(uint32_t nwork)
 // Planes of the listed chunks: CTA (x, y) takes the planes of item x that
 // fall to its warps of the item's gridDim.y * kDecodeWarps; the tables of
 // stream i at tabs[i].
-__global__ void __launch_bounds__(kDecodeThreads) k_decode(const CtaWork* __restrict__ work,
-                                                           const uint32_t* __restrict__ chunk_ids,
-                                                           const StreamDesc* __restrict__ sd,
-                                                           const DecodeTables* __restrict__ tabs,
-                                                           const uint16_t* __restrict__ cb_sym,
-                                                           const uint32_t* __restrict__ sub_off,
-                                                           const uint64_t* __restrict__ chunk_word_off,
-                                                           const uint32_t* __restrict__ payload,
-                                                           uint16_t* __restrict__ codes, bool halves)
+// LARGE: of at least kHalfWarpItems items; bound by instructions, four CTAs per
+// SM. Smaller launches are bound by latency and keep more in registers (72
+// against 62 and, before, spills): boxes of 384x384x256 f64 0.058 -> 0.048 ms.
+template <bool LARGE>
+__global__ void __launch_bounds__(kDecodeThreads, LARGE ? 4 : 3)
+    k_decode(const CtaWork* __restrict__ work, const uint32_t* __restrict__ chunk_ids,
+             const StreamDesc* __restrict__ sd, const DecodeTables* __restrict__ tabs,
+             const uint16_t* __restrict__ cb_sym, const uint32_t* __restrict__ sub_off,
+             const uint64_t* __restrict__ chunk_word_off, const uint32_t* __restrict__ payload,
+             uint16_t* __restrict__ codes)
 {
     extern __shared__ __align__(16) uint8_t decode_smem[];
     DecodeSmem& sm = *reinterpret_cast<DecodeSmem*>(decode_smem);
@@ -1122,7 +1163,7 @@ __global__ void __launch_bounds__(kDecodeThreads) k_decode(const CtaWork* __rest
     const StreamDesc s = sd[w.stream];
     const uint32_t P = s.C * s.C, np = w.count * s.C;
     uint32_t W = decode_lanes(P);
-    if (halves && P == kMaxPlane && s.code_off % 8 == 0 &&
+    if (LARGE && P == kMaxPlane && s.code_off % 8 == 0 &&
         32 * (s.word_cap - 4) < (uint64_t)kHalfWarpBits * s.nchunks * s.C)
         W = 16;
     if (blockIdx.y * kDecodeWarps * (32 / W) >= np) return;  // uniform per block
@@ -1368,10 +1409,10 @@ void launch_decode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, co
                    const uint32_t* payload, uint16_t* codes, cudaStream_t st)
 {
     if (!nwork) return;
-    cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecodeSmem));
-    const DecodeTables* t = static_cast<const DecodeTables*>(tables);
-    k_decode<<<dim3(nwork, decode_slices((uint32_t)nwork)), kDecodeThreads, sizeof(DecodeSmem), st>>>(
-        work, chunk_ids, sd, t, cb_sym, sub_off, chunk_word_off, payload, codes, nwork >= kHalfWarpItems);
+    auto* k = nwork >= kHalfWarpItems ? k_decode<true> : k_decode<false>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecodeSmem));
+    k<<<dim3(nwork, decode_slices((uint32_t)nwork)), kDecodeThreads, sizeof(DecodeSmem), st>>>(
+        work, chunk_ids, sd, static_cast<const DecodeTables*>(tables), cb_sym, sub_off, chunk_word_off, payload, codes);
 }
 
 size_t decode_tables_bytes() { return sizeof(DecodeTables); }
