@@ -320,10 +320,11 @@ __device__ __forceinline__ void encode_interior(const Acc& r, const EncodeIO<T>&
             if (code == qp.radius) {
                 ++center[b];
             } else {
-                hist_add(sh, wlo, wn, hist, b, code, 1u);
+                if (!kGatherZeros<T, FINEST> || code) hist_add(sh, wlo, wn, hist, b, code, 1u, center[b]);
                 if (code == 0) {
                     io.unpred_dense[(size_t)b * n + zw.cm] = d;
-                    atomicAdd(&io.unpred_cnt[(size_t)b * (geo.nchunks() + 1) + zw.chunk], 1u);
+                    if (kGatherZeros<T, FINEST>) center[b] += kOneZero;
+                    else atomicAdd(&io.unpred_cnt[(size_t)b * (geo.nchunks() + 1) + zw.chunk], 1u);
                 }
             }
         }
@@ -345,8 +346,32 @@ __device__ __forceinline__ void encode_interior(const Acc& r, const EncodeIO<T>&
     }
 }
 
+// A warp's unpredictable values since the last flush (at most ZB per lane and
+// stream, all of one layer of chunks): one atomic per chunk and stream.
+template <typename T>
+__device__ __forceinline__ void flush_zeros(const EncodeIO<T>& io, const LevelGeom& geo, int chunk,
+                                            uint32_t (*sh)[kSmemBins], int wlo, int wn, const HistArgs& hist,
+                                            uint32_t (&center)[7])
+{
+    uint32_t any = 0;
+#pragma unroll
+    for (int b = 0; b < 7; ++b) any |= center[b];
+    if (!__any_sync(0xffffffffu, any & kZeros)) return;
+    const uint32_t mask = __match_any_sync(0xffffffffu, chunk);
+    const bool first = (threadIdx.x & 31) == __ffs(mask) - 1;
+#pragma unroll
+    for (int b = 0; b < 7; ++b) {
+        const uint32_t c = __reduce_add_sync(mask, (center[b] & kZeros) / kOneZero);
+        center[b] &= ~kZeros;
+        if (first && c) {
+            hist_add(sh, wlo, wn, hist, b, 0, c, center[b]);
+            atomicAdd(&io.unpred_cnt[(size_t)b * (geo.nchunks() + 1) + chunk], c);
+        }
+    }
+}
+
 template <typename T, int PRED, bool FINEST, int LM, int ZB = kZSmall>
-__global__ void __launch_bounds__(BX* BY, LM == kLearnNone && sizeof(T) == 4 ? (FINEST ? 5 : 4) : 1) k_level_encode(EncodeIO<T> io, const T* __restrict__ R, LevelGeom geo,
+__global__ void __launch_bounds__(BX* BY, LM != kLearnNone ? 1 : sizeof(T) == 4 ? (FINEST ? 5 : 4) : FINEST ? 1 : 2) k_level_encode(EncodeIO<T> io, const T* __restrict__ R, LevelGeom geo,
                                                          QuantParams qp, HistArgs hist, LearnedArgs<T> la,
                                                          const __grid_constant__ CUtensorMap tmap, int use_tma,
                                                          const __grid_constant__ QuantTable qt)
@@ -399,6 +424,8 @@ __global__ void __launch_bounds__(BX* BY, LM == kLearnNone && sizeof(T) == 4 ? (
             if (valid)
                 encode_interior<T, PRED, FINEST>(r, io, geo, qp, lut, zw, fp, gp, sh, wlo, wn, hist, center,
                                                  use_qt ? qtab : nullptr, qt.r2);
+            if (kGatherZeros<T, FINEST> && (z + 1 == z1 || zw.lz + 1 == zw.C))
+                flush_zeros(io, geo, zw.chunk, sh, wlo, wn, hist, center);
             zw.next();
             fp += fstep;
             if constexpr (!FINEST) gp += 2 * gsy;
@@ -418,7 +445,7 @@ __global__ void __launch_bounds__(BX* BY, LM == kLearnNone && sizeof(T) == 4 ? (
 #pragma unroll
                 for (int b = 0; b < 7; ++b) {
                     if (q[b] == qp.radius) ++center[b];
-                    else hist_add(sh, wlo, wn, hist, b, q[b], 1u);
+                    else hist_add(sh, wlo, wn, hist, b, q[b], 1u, center[b]);
                 }
             });
         }
