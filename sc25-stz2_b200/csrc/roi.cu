@@ -111,7 +111,10 @@ __global__ void __launch_bounds__(256) k_roi_cells(const uint8_t* __restrict__ m
         v[0] = r(0);
 #pragma unroll
         for (int b = 0; b < 7; ++b) {
-            const T dq = q[b] ? recover<T>(q[b], qp) : __ldg(unpred_dense + (size_t)b * n + cm);
+            // (where a parity lies outside the window its chunk may not be
+            // decoded: the code is then whatever the buffer held, 0 even in a
+            // stream without unpredictable values, which has no list of them)
+            const T dq = q[b] || !unpred_dense ? recover<T>(q[b], qp) : __ldg(unpred_dense + (size_t)b * n + cm);
             v[b + 1] = A::add(dq, p[b]);
         }
 #pragma unroll

@@ -15,8 +15,8 @@ void set_last_error(const std::string& msg);
 constexpr int kMaxCodeLen = 24;
 // Fast decode table width (bits) of the GPU decoder.
 constexpr int kLutBits = 12;
-// Histogram window (bins around the radius) kept in shared memory and copied
-// to the host for codebook construction; codes outside it take a slow path.
+// Codes around the radius that a codebook looks at when a stream has no others
+// (the encoder flags the streams that do; they have every code looked at).
 constexpr int kHistWindow = 4096;
 // Planes of one coder work item: an item covers max(1, 128 / C) chunks of a
 // stream, i.e. up to 128 planes (the coder kernels split an item over
