@@ -712,6 +712,7 @@ __global__ void __launch_bounds__(kLaneThreads) k_encode(const CtaWork* __restri
 // bits 16-31 (mod 2^16); else the symbol in bits 16-31 (its canonical index
 // where the stream decodes by index).
 constexpr uint32_t kLutRun = 0x100u, kLutLong = 0x200u;
+constexpr uint32_t kNoIndex = 0xffffu;  // a plane's entry without a literal, where the stream decodes by index
 struct DecodeTables {
     uint32_t lut[1 << kLutBits];
     // per code length: limit (codes of up to that length lie below it, as
@@ -771,8 +772,10 @@ __global__ void __launch_bounds__(kBuildThreads) k_build_tables(const StreamDesc
             if (l <= kLutBits) mass += cnt[l] << (kLutBits - l);
         }
         t.max_len = longest;
-        // more than one symbol in 128 has a long code
-        by_index = t.by_index = (1u << kLutBits) - mass > (1u << kLutBits) / 128 && longest > kLutBits;
+        // more than one symbol in 128 has a long code; with run symbols an
+        // entry can stay without a literal, so kNoIndex must not be an index
+        by_index = t.by_index = (1u << kLutBits) - mass > (1u << kLutBits) / 128 && longest > kLutBits &&
+                                (s.run_n == 0 || s.n_used <= kNoIndex);
     }
     __syncthreads();
     if (tid <= kMaxCodeLen)
@@ -817,7 +820,6 @@ constexpr int kDecodeWarps = 8;
 constexpr int kDecodeThreads = 32 * kDecodeWarps;
 constexpr uint32_t kMaxPlane = 1024;    // planes of up to this many codes fit the shared buffers
 constexpr uint32_t kStageWords = 512;   // payload words of the planes a warp decodes at a time
-constexpr uint32_t kNoIndex = 0xffffu;  // a plane's entry without a literal (by_index)
 
 struct DecodeSmem {
     uint32_t lut[1 << kLutBits];
