@@ -235,19 +235,6 @@ struct XferEvents {
             if (x) cudaEventDestroy(x);
     }
 };
-
-// On an early return (a failed CUDA call mid-loop), waits for the copies
-// already queued on the stream, so the next host-buffer call never refills a
-// staging chunk that a DMA still reads or writes. The wait's own status is
-// ignored: the caller already reports the first error.
-struct DrainOnExit {
-    cudaStream_t st;
-    bool done = false;
-    ~DrainOnExit()
-    {
-        if (!done) cudaStreamSynchronize(st);
-    }
-};
 }  // namespace
 
 stz_status copy_to_host(stz_context* ctx, void* dst, const void* src_dev, size_t n)
@@ -413,6 +400,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
 {
     Lap lap("compress");
     cudaStream_t st = ctx->st;
+    DrainOnExit drain{st, ctx->st_copy, ctx->st_side};
     const Geometry g = make_geometry(nx, ny, nz, o.chunk_high, o.chunk_low, o.radius);
     const int K = g.K, R2 = 2 * o.radius;
     const int nstreams = 7 * K;
@@ -891,6 +879,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     }
     lap.mark("parse check");
     *out = so;
+    drain.done = true;  // st_copy was waited for, and behind it the last kernels of st and st_side
     return STZ_OK;
 }
 
@@ -1068,6 +1057,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
     // decoding) runs while the next batch is being zstd-decoded.
     const size_t o_tab = align256(total), dev_total = o_tab + (size_t)nstreams * decode_tables_bytes();
     STZ_CUDA(p.stage->ensure(dev_total));
+    DrainOnExit drain{ctx->st, ctx->st_copy, ctx->st_dec};
     STZ_CUDA(cudaMemcpyAsync(p.stage->p, hs, o_pl, cudaMemcpyHostToDevice, ctx->st));
     uint8_t* ds = p.stage->as<uint8_t>();
     p.d_sd = (StreamDesc*)(ds + o_sd);
@@ -1116,11 +1106,6 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
             for (cudaEvent_t x : e) cudaEventDestroy(x);
         }
     } ev;
-    auto sync_both = [&]() {
-        cudaStreamSynchronize(ctx->st_copy);
-        cudaStreamSynchronize(ctx->st_dec);
-        cudaStreamSynchronize(ctx->st);
-    };
     std::vector<size_t> bjobs;
     for (const DecodeBatch& B : batches) {
         // the batch's frames: whole streams, or layers [l0, l1) of each
@@ -1135,10 +1120,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
             if (J.stored == J.raw) stream_copy(J.dst, J.src, J.raw);
             else if (!decode_frame(J.src, J.stored, J.raw, J.dst)) bad = 3;
         });
-        if (bad) {
-            sync_both();
-            STZ_FAIL(STZ_ERR_ZSTD, "payload frame does not decode");
-        }
+        if (bad) STZ_FAIL(STZ_ERR_ZSTD, "payload frame does not decode");
         cudaEvent_t e = nullptr;
         cudaError_t ce = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
         if (ce == cudaSuccess) ev.e.push_back(e);
@@ -1157,22 +1139,14 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         }
         if (ce == cudaSuccess) ce = cudaEventRecord(e, ctx->st_copy);
         if (ce == cudaSuccess && !on_batch && B.s1 == nstreams) ce = cudaStreamWaitEvent(ctx->st, e, 0);
-        if (ce != cudaSuccess) {
-            sync_both();
-            STZ_CUDA(ce);
-        }
-        if (on_batch) {
-            const stz_status st = (*on_batch)(B, e);
-            if (st != STZ_OK) {
-                sync_both();
-                return st;
-            }
-        }
+        STZ_CUDA(ce);
+        if (on_batch) STZ_TRY((*on_batch)(B, e));
     }
     lap.mark("payload frames + h2d");
     STZ_CUDA(cudaStreamSynchronize(ctx->st_copy));  // the pinned staging buffer is reused by the next call
     STZ_CUDA(cudaStreamSynchronize(ctx->st_dec));
     STZ_CUDA(cudaStreamSynchronize(ctx->st));
+    drain.done = true;
     lap.mark("host->device");
     return STZ_OK;
 }

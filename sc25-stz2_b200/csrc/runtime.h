@@ -102,6 +102,24 @@ struct PinBuf {
     }
 };
 
+// On an early return (a failed CUDA call or allocation), waits for the work
+// already queued on the streams: the next call writes the pinned buffers and
+// the descriptors that it still reads. The waits' own status is ignored: the
+// caller already reports the first error.
+struct DrainOnExit {
+    cudaStream_t st[3];
+    bool done = false;
+    explicit DrainOnExit(cudaStream_t a, cudaStream_t b = nullptr, cudaStream_t c = nullptr) : st{a, b, c} {}
+    DrainOnExit(const DrainOnExit&) = delete;
+    DrainOnExit& operator=(const DrainOnExit&) = delete;
+    ~DrainOnExit()
+    {
+        if (done) return;
+        for (cudaStream_t s : st)
+            if (s) cudaStreamSynchronize(s);
+    }
+};
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Device-resident decode inputs of levels 1..kmax of one stream object.
