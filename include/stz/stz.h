@@ -468,6 +468,11 @@ stz_status stz_debug_codebook(const uint32_t* hist, int nbins, uint16_t* sym, ui
  * *run_base (0: no runs). Host only. */
 stz_status stz_debug_run_slots(const uint32_t* hist, int nbins, int plane, uint32_t* run_base, uint32_t* run_n);
 
+/* Sets the device word that a level kernel sets when an MMA of the learned
+ * network did not complete in time, as if one had: the next call on the device
+ * that uses a learned correction fails with STZ_ERR_CUDA. */
+stz_status stz_debug_learned_fail(stz_context* ctx);
+
 #ifdef __cplusplus
 }
 #endif

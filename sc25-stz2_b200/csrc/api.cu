@@ -607,6 +607,11 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaEventRecord(named[EvLevels], st));
     STZ_CUDA(cudaStreamWaitEvent(st, named[EvUp], 0));
 
+    // A learned level whose MMA wait gave up has left codes unwritten and
+    // uncounted: the coder must not read them. (A lost tile load leaves wrong
+    // values, but codes and counts that agree; its flag is read at the end.)
+    if (M && M->mask && learned_tc_error_take(st))
+        STZ_FAIL(STZ_ERR_CUDA, "learned correction: a tensor-core MMA did not complete in time");
     // The rest of the device's work, from run symbols to payload words, goes
     // out at once: nothing of it waits for the host.
     if (rs_any) {
@@ -864,8 +869,6 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     }
     STZ_CUDA(cudaStreamSynchronize(ctx->st_copy));  // every group's copy (the payload buffer is reused next call)
     if (level_error_take()) STZ_FAIL(STZ_ERR_CUDA, "level kernel: a TMA tile load did not complete in time");
-    if (M && M->mask && learned_tc_error_take(st))
-        STZ_FAIL(STZ_ERR_CUDA, "learned correction: a tensor-core MMA did not complete in time");
     lap.mark("encode + copy + zstd");
     auto* so = new (std::nothrow) stz_stream();
     if (!so) STZ_FAIL(STZ_ERR_NOMEM, "out of host memory");

@@ -115,3 +115,11 @@ extern "C" stz_status stz_debug_learned_infer(stz_context* ctx, const int8_t* xq
     if (e) STZ_FAIL(STZ_ERR_CUDA, "tensor-core inference: an MMA did not complete in time");
     return STZ_OK;
 }
+
+extern "C" stz_status stz_debug_learned_fail(stz_context* ctx)
+{
+    if (!ctx) STZ_FAIL(STZ_ERR_ARG, "null pointer");
+    STZ_TRY(enter(ctx));
+    STZ_CUDA(learned_tc_error_raise(ctx->st));
+    return STZ_OK;
+}

@@ -82,6 +82,13 @@ uint32_t learned_tc_error_take(cudaStream_t st)
     return v;
 }
 
+cudaError_t learned_tc_error_raise(cudaStream_t st)
+{
+    const uint32_t one = 1;
+    const cudaError_t e = cudaMemcpyToSymbolAsync(g_learned_tc_error, &one, 4, 0, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 namespace {
 
 template <typename T>

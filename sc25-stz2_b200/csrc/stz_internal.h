@@ -66,8 +66,10 @@ struct LearnedArgs {
 };
 
 // Nonzero when a tensor-core MMA of the learned network did not complete in
-// time (a bounded wait gave up); read and cleared by learned_tc_error_take.
+// time (a bounded wait gave up); read and cleared by learned_tc_error_take,
+// set from the host by learned_tc_error_raise (tests).
 uint32_t learned_tc_error_take(cudaStream_t st);
+cudaError_t learned_tc_error_raise(cudaStream_t st);
 
 // The level kernels' TMA tile-load error word: level_error_init maps it for
 // the current device (once per context); level_error_take returns whether a

@@ -130,6 +130,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
     lib.stz_debug_mlp_grad.argtypes = [vp, vp, vp, vp, sz, C.c_double, C.c_double, C.c_double, C.c_int,
                                        C.POINTER(C.c_double), vp, C.POINTER(C.c_double)]
     lib.stz_debug_learned_infer.argtypes = [vp, vp, sz, vp, C.c_int, vp]
+    lib.stz_debug_learned_fail.argtypes = [vp]
     lib.stz_model_parse.argtypes = [vp, sz, C.POINTER(vp)]
     lib.stz_model_bytes.argtypes = [vp, C.POINTER(vp), C.POINTER(sz)]
     lib.stz_model_free.argtypes = [vp]
