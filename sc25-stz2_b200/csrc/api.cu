@@ -826,12 +826,12 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     }
     // each stream header is built by the pool job that compresses it (the
     // finest streams', the largest, first)
-    auto build_header = [&](size_t s) {
+    auto build_header = [&](size_t s) -> bool {
         const StreamDesc& d = sd[s];
-        build_stream_header(parts[s], ctx->arena, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base, d.run_n,
-                            unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
-                            h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
-                            (int)d.C);
+        return build_stream_header(parts[s], ctx->arena, h_sym + d.cb_off, h_len + d.cb_off, d.n_used, d.run_base,
+                                   d.run_n, unpred_off[s + 1] - unpred_off[s], ul + unpred_off[s] * elem, elem,
+                                   h_ucnt + d.chunk_base, choff + d.chunk_base, subo + d.sub_base, (int)d.nchunks,
+                                   (int)d.C);
     };
     ctx->arena.reset();
     ContainerWriter cw(h, parts, *ctx->pool, ctx->arena);
@@ -870,7 +870,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaStreamSynchronize(ctx->st_copy));  // every group's copy (the payload buffer is reused next call)
     if (level_error_take()) STZ_FAIL(STZ_ERR_CUDA, "level kernel: a TMA tile load did not complete in time");
     lap.mark("encode + copy + zstd");
-    auto* so = new (std::nothrow) stz_stream();
+    auto* so = cw.out_of_memory() ? nullptr : new (std::nothrow) stz_stream();
     if (!so) STZ_FAIL(STZ_ERR_NOMEM, "out of host memory");
     so->bytes = cw.finish(coarsest.data(), levels);
     lap.mark("container");

@@ -457,7 +457,7 @@ struct Reader {
 
 }  // namespace
 
-void build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
+bool build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
                          uint32_t run_base, uint32_t run_n, uint64_t n_unpred, const void* unpred, size_t elem,
                          const uint32_t* unpred_count, const uint64_t* chunk_word_off, const uint32_t* sub_off,
                          int nchunks, int C)
@@ -472,7 +472,7 @@ void build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, 
     p.hdr_n = 4 + 3 * (size_t)n_used + 4 + 4 + 8 + n_unpred * elem + 4 * (size_t)nchunks + 8 * ((size_t)nchunks + 1) + 1 +
               (size_t)nchunks * (C - 1) * width;
     uint8_t* dst = p.hdr.take(arena, p.hdr_n);
-    if (!dst) throw std::bad_alloc();
+    if (!dst) return false;
     auto put = [&](const void* v, size_t n) {
         if (n) std::memcpy(dst, v, n);
         dst += n;
@@ -498,6 +498,7 @@ void build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, 
             }
             dst += width;
         }
+    return true;
 }
 
 bool parse_stream_header(const uint8_t* raw, size_t n, int nchunks, int C, size_t elem, int version,
@@ -657,7 +658,7 @@ ContainerWriter::ContainerWriter(const FileHeader& h, std::vector<StreamParts>& 
 
 void ContainerWriter::compress_groups(size_t ngroups, const std::function<size_t(size_t, int)>& group_of_frame,
                                       const std::function<void(size_t)>& wait_group,
-                                      const std::function<void(size_t)>& build_header)
+                                      const std::function<bool(size_t)>& build_header)
 {
     // group by group, largest frames first inside a group (headers not built
     // yet: later streams, the finer levels, first): the pool's threads move
@@ -696,7 +697,10 @@ void ContainerWriter::compress_groups(size_t ngroups, const std::function<size_t
         if (trace) j_go[k] = since(f0);
         if (!frames_[order[k]].payload) {
             const size_t st = stream_of[order[k]];
-            build_header(st);
+            if (!build_header(st)) {
+                out_of_memory_ = true;
+                return;
+            }
             frames_[order[k]].src = parts_[st].hdr.p;
             frames_[order[k]].n = parts_[st].hdr_n;
         }
@@ -719,7 +723,10 @@ void ContainerWriter::compress_groups(size_t ngroups, const std::function<size_t
         if (try_zstd) {
             const size_t cap = ZSTD_compressBound(f.n);
             uint8_t* const z = f.out.take(arena_, cap);
-            if (!z) throw std::bad_alloc();
+            if (!z) {
+                out_of_memory_ = true;
+                return;
+            }
             const size_t c = zstd_compress(z, cap, f.src, f.n, level);
             if (!ZSTD_isError(c) && c < f.n) {
                 f.stored = c;

@@ -222,8 +222,8 @@ struct StreamParts {
     int layers = 0, chunks_per_layer = 0;
 };
 
-// The stream's header bytes into p.hdr, p.hdr_n.
-void build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
+// The stream's header bytes into p.hdr, p.hdr_n; false without memory.
+bool build_stream_header(StreamParts& p, HostArena& arena, const uint16_t* sym, const uint8_t* len, uint32_t n_used,
                          uint32_t run_base, uint32_t run_n, uint64_t n_unpred, const void* unpred, size_t elem,
                          const uint32_t* unpred_count, const uint64_t* chunk_word_off, const uint32_t* sub_off,
                          int nchunks, int C);
@@ -246,10 +246,12 @@ public:
     // [0, ngroups) (anything else: not compressed by this call); a thread
     // calls wait_group(g) before each frame of group g. build_header: the job
     // of stream s's header frame first calls it to fill parts[s].hdr, so each
-    // header is built and compressed by one job.
+    // header is built and compressed by one job (false: no memory for it).
     void compress_groups(size_t ngroups, const std::function<size_t(size_t, int)>& group_of_frame,
                          const std::function<void(size_t)>& wait_group,
-                         const std::function<void(size_t)>& build_header);
+                         const std::function<bool(size_t)>& build_header);
+    // A job found no memory: there is no container (pool threads do not throw).
+    bool out_of_memory() const { return out_of_memory_; }
     Bytes finish(const void* coarsest, const std::vector<LevelDir>& levels);
 
 private:
@@ -268,6 +270,7 @@ private:
     HostArena& arena_;
     std::vector<Frame> frames_;
     std::vector<size_t> first_;  // first frame of each stream (+ end)
+    std::atomic<bool> out_of_memory_{false};
     std::atomic<int64_t> busy_ns_{0};
     int64_t wall_ns_ = 0;
 };

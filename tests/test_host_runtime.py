@@ -61,3 +61,49 @@ int main()
 }
 """)
     assert out.strip() == "123||123|4"
+
+
+def test_a_container_job_without_memory_does_not_throw(tmp_path):
+    """Frames are built and compressed on pool threads, where an exception
+    ends the process: a job that gets no memory is reported instead, for
+    headers and for compressed payload frames."""
+    out = run(tmp_path, r"""
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include "host.h"
+static std::atomic<size_t> limit{SIZE_MAX};
+void* operator new[](size_t n, const std::nothrow_t&) noexcept { return n > limit ? nullptr : std::malloc(n); }
+void operator delete[](void* p) noexcept { std::free(p); }
+void operator delete[](void* p, size_t) noexcept { std::free(p); }
+static int once(bool header, bool payload)
+{
+    using namespace stz;
+    const int layers = 3, C = 4;
+    const size_t per = 40000;  // words a layer; zeros, so each frame is worth compressing
+    std::vector<uint32_t> words(layers * per, 0);
+    std::vector<uint64_t> off(layers + 1);
+    for (int i = 0; i <= layers; ++i) off[i] = i * per;
+    std::vector<uint32_t> sub(layers * C, 0), unpred(layers, 0);
+    FileHeader h{};
+    h.zstd_level = 3;
+    std::vector<StreamParts> parts(5);
+    for (auto& p : parts) p.words = words.data(), p.chunk_word_off = off.data(), p.layers = layers, p.chunks_per_layer = 1;
+    ThreadPool pool(4);
+    HostArena arena;  // empty: every block is its own
+    ContainerWriter w(h, parts, pool, arena);
+    const uint16_t sym[2] = {1, 2};
+    const uint8_t len[2] = {1, 1};
+    std::vector<uint8_t> values(header ? 200000 : 8);
+    limit = header || payload ? 100000 : SIZE_MAX;
+    w.compress_groups(1, [&](size_t, int layer) -> size_t { return layer < 0 || payload ? 0 : SIZE_MAX; }, [](size_t) {},
+                      [&](size_t s) {
+                          return build_stream_header(parts[s], arena, sym, len, 2, 0, 0, values.size(), values.data(), 1,
+                                                     unpred.data(), off.data(), sub.data(), layers, C);
+                      });
+    limit = SIZE_MAX;
+    return w.out_of_memory();
+}
+int main() { std::printf("%d%d%d\n", once(false, false), once(true, false), once(false, true)); }
+""", ["host.cpp"], ["-l:libzstd.so.1"])
+    assert out.strip() == "011"
