@@ -836,12 +836,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     ctx->arena.reset();
     ContainerWriter cw(h, parts, *ctx->pool, ctx->arena);
     std::atomic<int> ev_err{0};
-    // One thread waits for a group's copy, the others for that thread (0: not
-    // waited for, 1: being waited for, 2: complete): concurrent calls from the
-    // pool's threads serialize in the driver, and an event that blocks its
-    // waiter wakes it 0.35 ms late.
-    std::unique_ptr<std::atomic<int>[]> copied(new std::atomic<int>[ngroups]);
-    for (size_t i = 0; i < ngroups; ++i) copied[i].store(0);
+    SharedWaits copied(ngroups);
     // zstd groups: every stream header first (nothing to wait for), then
     // the payload of encode group g after its copy (event g)
     cw.compress_groups(
@@ -853,14 +848,9 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         },
         [&](size_t g) {
             if (g == 0) return;
-            std::atomic<int>& c = copied[g - 1];
-            int none = 0;
-            if (c.compare_exchange_strong(none, 1)) {
+            copied.wait(g - 1, [&]() {
                 if (cudaEventSynchronize(ev.e[g - 1]) != cudaSuccess) ev_err = 1;
-                c.store(2, std::memory_order_release);
-            } else {
-                while (c.load(std::memory_order_acquire) != 2) std::this_thread::yield();
-            }
+            });
         },
         build_header);
     if (ev_err) {  // reports the device error

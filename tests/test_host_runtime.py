@@ -107,3 +107,38 @@ static int once(bool header, bool payload)
 int main() { std::printf("%d%d%d\n", once(false, false), once(true, false), once(false, true)); }
 """, ["host.cpp"], ["-l:libzstd.so.1"])
     assert out.strip() == "011"
+
+
+def test_threads_that_wait_for_another_do_not_use_a_core(tmp_path):
+    """Seven threads wait 0.4 s for what the eighth waits for: each thing is
+    waited for once, is done when wait returns, and the process uses a fraction
+    of that time (polling threads would use seven times it)."""
+    out = run(tmp_path, r"""
+#include <cstdio>
+#include <sys/resource.h>
+#include "host.h"
+int main()
+{
+    stz::SharedWaits w(2);
+    std::atomic<int> calls{0}, early{0};
+    std::atomic<bool> done[2] = {{false}, {false}};
+    std::vector<std::thread> t;
+    for (int k = 0; k < 8; ++k)
+        t.emplace_back([&] {
+            for (size_t i = 0; i < 2; ++i) {
+                w.wait(i, [&] {
+                    ++calls;
+                    std::this_thread::sleep_for(std::chrono::milliseconds(200));
+                    done[i] = true;
+                });
+                if (!done[i]) ++early;
+            }
+        });
+    for (auto& x : t) x.join();
+    rusage r;
+    getrusage(RUSAGE_SELF, &r);
+    const double cpu = r.ru_utime.tv_sec + r.ru_stime.tv_sec + 1e-6 * (r.ru_utime.tv_usec + r.ru_stime.tv_usec);
+    std::printf("%d %d %d\n", (int)calls, (int)early, cpu < 0.2);
+}
+""")
+    assert out.split() == ["2", "0", "1"]
