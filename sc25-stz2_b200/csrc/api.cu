@@ -557,13 +557,16 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         max_chunks = std::max(max_chunks, sd[s].nchunks);
     }
     const uint64_t cb_cap = cb_items[nstreams];
-    // sd | work | ids | codebook scratch offsets
-    const size_t o_work = align256(sd.size() * sizeof(StreamDesc));
+    // sd | sd | work | ids | codebook scratch offsets: the codebook kernels
+    // write into the first descriptors; the second stay as they are, for the
+    // gather of unpredictable values beside them on another stream
+    const size_t o_sd1 = align256(sd.size() * sizeof(StreamDesc)), o_work = 2 * o_sd1;
     const size_t o_ids = align256(o_work + work.size() * sizeof(CtaWork));
     const size_t o_cbi = align256(o_ids + ids.size() * 4), up_bytes = align256(o_cbi + cb_items.size() * 8);
     STZ_CUDA(ctx->h_stage.ensure(up_bytes));
     uint8_t* hs = ctx->h_stage.as<uint8_t>();
     std::memcpy(hs, sd.data(), sd.size() * sizeof(StreamDesc));
+    std::memcpy(hs + o_sd1, sd.data(), sd.size() * sizeof(StreamDesc));
     std::memcpy(hs + o_work, work.data(), work.size() * sizeof(CtaWork));
     std::memcpy(hs + o_ids, ids.data(), ids.size() * 4);
     std::memcpy(hs + o_cbi, cb_items.data(), cb_items.size() * 8);
@@ -573,6 +576,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaMemsetAsync(ctx->rstats.p, 0, (size_t)nstreams * kRunStats * 8, sc));
     uint8_t* dstage = ctx->sd.as<uint8_t>();
     StreamDesc* d_sd = (StreamDesc*)dstage;
+    const StreamDesc* d_sd1 = (const StreamDesc*)(dstage + o_sd1);
     const CtaWork* d_work = (const CtaWork*)(dstage + o_work);
     const uint32_t* d_ids = (const uint32_t*)(dstage + o_ids);
     const uint64_t* d_cbi = (const uint64_t*)(dstage + o_cbi);
@@ -716,8 +720,8 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
         {
             KScope ks(ctx, "k_unpred_move", 1, su);
             launch_unpred_move<T>(true, unpred_little(sd, uwork.data(), uwork.size()), ctx->uwork.as<UnpredWork>(),
-                                  (int)uwork.size(), d_sd,
-                                  ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(), ctx->ulist.as<T>(), su);
+                                  (int)uwork.size(), d_sd1, ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(),
+                                  ctx->ulist.as<T>(), su);
         }
         STZ_CUDA(cudaGetLastError());
         STZ_CUDA(cudaMemcpyAsync(ht + t_ul, ctx->ulist.p, total_unpred * elem, cudaMemcpyDeviceToHost, su));
