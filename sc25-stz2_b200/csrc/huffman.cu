@@ -1226,26 +1226,27 @@ __global__ void __launch_bounds__(kDecodeThreads, 3) k_decode_dyn(const uint8_t*
 // shared memory, so that the moves are spread over all threads wherever the
 // zeros lie (along a front, most codes of a chunk are zero). Bound by latency.
 // Launches with chunks of more than 4096 codes take 1024 threads a chunk (one
-// mask each for 32^3), the others 256, of which one warp does a chunk of up
-// to 4096 alone. Before (a thread read its 32 codes one by one, twice, and
-// moved its own values) and now: 512^3 f32 at 1e-4, decode, 0.25 ->
-// 0.059 ms; 384x384x256 f64 fronts at 1e-6, decode, 0.32 -> 0.15 ms; a box of
-// them 21 -> 11.6 us; 336x272x208 f32 with chunks of 8, 0.14 -> 0.079 ms.
+// mask each for 32^3; a chunk of up to 1024 codes is one warp's work), the
+// others a warp a chunk, in a CTA of its own (336x272x208 f32 fronts at 1e-5
+// with chunks of 8, decode, 0.079 ms with eight-warp CTAs, of which one worked,
+// and 0.065 so). Before (a thread read its 32 codes one by one, twice, and
+// moved its own values) and now: 512^3 f32 at 1e-4, decode, 0.25 -> 0.059 ms;
+// 384x384x256 f64 fronts at 1e-6, decode, 0.32 -> 0.15 ms; a box of them 21 ->
+// 11 us; 336x272x208 f32 with chunks of 8, 0.14 -> 0.065 ms.
 constexpr uint32_t kUnpredSmall = 4096;
 template <uint32_t THREADS, uint32_t TILES>
 struct UnpredShape {
     static constexpr uint32_t threads = THREADS;
-    static constexpr uint32_t tiles = TILES;                    // masks per thread
-    static constexpr uint32_t warp = 32 * 32 * TILES;           // codes a warp holds
-    static constexpr uint32_t span = warp * (THREADS / 32);     // codes the CTA holds
-    static constexpr uint32_t list = THREADS == 1024 ? span : warp;  // positions listed at a time
+    static constexpr uint32_t tiles = TILES;                 // masks per thread
+    static constexpr uint32_t warp = 32 * 32 * TILES;        // codes a warp holds
+    static constexpr uint32_t span = warp * (THREADS / 32);  // codes the CTA holds
 };
 using UnpredBig = UnpredShape<1024, 1>;
-using UnpredLittle = UnpredShape<256, 4>;
+using UnpredLittle = UnpredShape<32, kUnpredSmall / 1024>;
 template <class S>
 struct UnpredSmem {
     uint32_t wsum[S::threads / 32];
-    uint16_t pos[S::list];
+    uint16_t pos[S::span];
 };
 
 template <class S, typename T, bool GATHER>
@@ -1255,7 +1256,7 @@ __device__ __forceinline__ void unpred_move_one(const UnpredWork& uw, const Stre
 {
     const StreamDesc s = sd[uw.stream];
     const uint32_t vol = s.C * s.C * s.C, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const bool alone = vol <= S::warp;  // one warp's work
+    const bool alone = S::threads == 32 || vol <= S::warp;  // one warp's work
     if (alone && wid) return;
     const uint32_t threads = alone ? 32u : S::threads;
     auto sync = [&]() {
@@ -1304,25 +1305,22 @@ __device__ __forceinline__ void unpred_move_one(const UnpredWork& uw, const Stre
                 all += v;
             }
         }
-        for (uint32_t l0 = 0; l0 < all; l0 += S::list) {
 #pragma unroll
-            for (uint32_t t = 0; t < S::tiles; ++t) {
-                uint32_t r = r0 + rank[t] - l0;
-                for (uint32_t mm = m[t]; mm; mm &= mm - 1, ++r)
-                    if (r < S::list) sm.pos[r] = (uint16_t)(w0 + t * 1024 + lane * 32 + (__ffs(mm) - 1));
-            }
-            sync();
-            for (uint32_t k = threadIdx.x; k < min(all - l0, S::list); k += threads) {
-                const uint64_t r = before + l0 + k;
-                if (r >= uw.count) break;
-                const size_t d = base + at + sm.pos[k];
-                if (GATHER) list[uw.list_off + r] = dense[d];
-                else dense[d] = list[uw.list_off + r];
-            }
-            sync();  // the list is written again
+        for (uint32_t t = 0; t < S::tiles; ++t) {
+            uint32_t r = r0 + rank[t];
+            for (uint32_t mm = m[t]; mm; mm &= mm - 1, ++r)
+                sm.pos[r] = (uint16_t)(w0 + t * 1024 + lane * 32 + (__ffs(mm) - 1));
         }
+        sync();
+        for (uint32_t k = threadIdx.x; k < all; k += threads) {
+            const uint64_t r = before + k;
+            if (r >= uw.count) break;
+            const size_t d = base + at + sm.pos[k];
+            if (GATHER) list[uw.list_off + r] = dense[d];
+            else dense[d] = list[uw.list_off + r];
+        }
+        sync();  // the list and wsum are written again
         before += all;
-        if (!alone) __syncthreads();  // so is wsum
     }
 }
 
