@@ -301,7 +301,11 @@ def _pct(v, q):
 def serve_load(srv, sid, dims_xyz, K, rate, seconds, gen, seed):
     """Open-loop Poisson load: a producer thread submits at the arrival times,
     a consumer waits for each ticket and releases its output. Latency is the
-    server's own submit -> result-complete time."""
+    server's own submit -> result-complete time. Python's collector is held off
+    while the load runs: a full collection stops the producer for 40 to 60 ms,
+    and the requests that fall due meanwhile then arrive in one burst (at 50k a
+    second, p99 20 to 27 ms with it and 1.1 to 1.2 without)."""
+    import gc
     import threading
 
     rng = np.random.default_rng(seed)
@@ -331,25 +335,32 @@ def serve_load(srv, sid, dims_xyz, K, rate, seconds, gen, seed):
     lat = {"box": [], "slice": [], "level": []}
     batch_sizes, out_bytes, queue, order, trace = [], 0, [], [], []
     th = threading.Thread(target=producer)
+    collecting = gc.isenabled()
+    gc.collect()
+    gc.disable()
     t0 = time.perf_counter()
     th.start()
-    for i in range(n):
-        ready.acquire()
-        if err:
-            break
-        res = srv.wait(tickets[i])
-        srv.release(tickets[i])
-        if res.status != 0:
-            err.append(f"status {res.status}")
-            break
-        lat[reqs[i][0]].append(res.latency_ms)
-        order.append(res.latency_ms)
-        queue.append(res.queue_ms)
-        trace.append((arrivals[i], res.queue_ms, res.latency_ms, res.batch, res.batch_size))
-        batch_sizes.append(res.batch_size)
-        out_bytes += res.nbytes
-    wall = time.perf_counter() - t0
-    th.join()
+    try:
+        for i in range(n):
+            ready.acquire()
+            if err:
+                break
+            res = srv.wait(tickets[i])
+            srv.release(tickets[i])
+            if res.status != 0:
+                err.append(f"status {res.status}")
+                break
+            lat[reqs[i][0]].append(res.latency_ms)
+            order.append(res.latency_ms)
+            queue.append(res.queue_ms)
+            trace.append((arrivals[i], res.queue_ms, res.latency_ms, res.batch, res.batch_size))
+            batch_sizes.append(res.batch_size)
+            out_bytes += res.nbytes
+        wall = time.perf_counter() - t0
+    finally:
+        th.join()
+        if collecting:
+            gc.enable()
     if err:
         return {"error": err[0]}
     allv = [x for v in lat.values() for x in v]
