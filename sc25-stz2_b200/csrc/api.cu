@@ -719,7 +719,7 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
                                  cudaMemcpyHostToDevice, su));
         {
             KScope ks(ctx, "k_unpred_move", 1, su);
-            launch_unpred_move<T>(true, unpred_little(sd, uwork.data(), uwork.size()), ctx->uwork.as<UnpredWork>(),
+            launch_unpred_move<T>(true, unpred_codes_most(sd, uwork.data(), uwork.size()), ctx->uwork.as<UnpredWork>(),
                                   (int)uwork.size(), d_sd1, ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(),
                                   ctx->ulist.as<T>(), su);
         }
@@ -1172,7 +1172,7 @@ stz_status decode_chunks(stz_context* ctx, const Prepared& p, const std::vector<
     }
     if (!uwork.empty()) {
         KScope ks(ctx, "k_unpred_move");
-        launch_unpred_move<T>(false, unpred_little(p.sd, uwork.data(), uwork.size()), (const UnpredWork*)(dw + o_u),
+        launch_unpred_move<T>(false, unpred_codes_most(p.sd, uwork.data(), uwork.size()), (const UnpredWork*)(dw + o_u),
                               (int)uwork.size(), p.d_sd,
                               ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(), (T*)p.d_ulist, ctx->st);
     }
@@ -1225,7 +1225,7 @@ struct DecodePipe {
     bool planned = false;
     size_t next_batch = 0;
     std::vector<size_t> wfirst, ufirst;  // per batch: first work / unpredictable item (+ end)
-    std::vector<bool> ulittle;           // per batch: unpred_little of its items
+    std::vector<uint32_t> umost;         // per batch: unpred_codes_most of its items
     size_t o_w = 0, o_i = 0, o_u = 0;
     int next_level = 1, cur = 0;
     int fin_bricks = 0, fin_done = 0;  // the finest level's z-bricks, and those launched
@@ -1278,7 +1278,7 @@ struct DecodePipe {
         wfirst[batches.size()] = work.size();
         ufirst[batches.size()] = uw.size();
         for (size_t bi = 0; bi < batches.size(); ++bi)
-            ulittle.push_back(unpred_little(p.sd, uw.data() + ufirst[bi], ufirst[bi + 1] - ufirst[bi]));
+            umost.push_back(unpred_codes_most(p.sd, uw.data() + ufirst[bi], ufirst[bi + 1] - ufirst[bi]));
         o_w = 0, o_i = align256(work.size() * sizeof(CtaWork));
         o_u = align256(o_i + ids.size() * 4);
         const size_t total = align256(o_u + uw.size() * sizeof(UnpredWork));
@@ -1346,7 +1346,7 @@ struct DecodePipe {
         }
         if (u1 > u0) {
             KScope ks(ctx, "k_unpred_move", 1, sd);
-            launch_unpred_move<T>(false, ulittle[bi], (const UnpredWork*)(dw + o_u) + u0, (int)(u1 - u0), p.d_sd,
+            launch_unpred_move<T>(false, umost[bi], (const UnpredWork*)(dw + o_u) + u0, (int)(u1 - u0), p.d_sd,
                                   ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(), (T*)p.d_ulist, sd);
         }
         const ParsedStream& ps = s->dir;
@@ -1596,7 +1596,7 @@ stz_status decompress_box_dev(stz_context* ctx, stz_stream* s, const int64_t lo[
     }
     if (!uw.empty()) {
         KScope ks(ctx, "k_unpred_move");
-        launch_unpred_move<T>(false, unpred_little(p->sd, uw.data(), uw.size()), (const UnpredWork*)(dm + hd.o_uwork),
+        launch_unpred_move<T>(false, unpred_codes_most(p->sd, uw.data(), uw.size()), (const UnpredWork*)(dm + hd.o_uwork),
                               (int)uw.size(), p->d_sd,
                               ctx->codes.as<uint16_t>(), ctx->unpred_dense.as<T>(), (T*)p->d_ulist, ctx->st);
     }

@@ -1225,24 +1225,21 @@ __global__ void __launch_bounds__(kDecodeThreads, 3) k_decode_dyn(const uint8_t*
 // 16-byte loads, so the codes are read once. The positions go to a list in
 // shared memory, so that the moves are spread over all threads wherever the
 // zeros lie (along a front, most codes of a chunk are zero). Bound by latency.
-// Launches with chunks of more than 4096 codes take 1024 threads a chunk (one
-// mask each for 32^3; a chunk of up to 1024 codes is one warp's work), the
-// others a warp a chunk, in a CTA of its own (336x272x208 f32 fronts at 1e-5
-// with chunks of 8, decode, 0.079 ms with eight-warp CTAs, of which one worked,
-// and 0.065 so). Before (a thread read its 32 codes one by one, twice, and
+// A launch takes a thread for every 32 codes of its largest chunk: a warp, four
+// or 32 (in larger CTAs a chunk of up to 1024 codes is one warp's work, and a
+// chunk of more than 32768 takes several spans). With one warp for chunks of up
+// to 4096, a warp's lanes listed up to 128 zeros each: 128^3 f64 GRF at 1e-5,
+// half resolution, 0.030 -> 0.012 ms; 256^3 f64 fronts with chunks of 16, 0.14
+// -> 0.072. Before that (a thread read its 32 codes one by one, twice, and
 // moved its own values) and now: 512^3 f32 at 1e-4, decode, 0.25 -> 0.059 ms;
-// 384x384x256 f64 fronts at 1e-6, decode, 0.32 -> 0.15 ms; a box of them 21 ->
-// 11 us; 336x272x208 f32 with chunks of 8, 0.14 -> 0.065 ms.
-constexpr uint32_t kUnpredSmall = 4096;
-template <uint32_t THREADS, uint32_t TILES>
+// 384x384x256 f64 fronts at 1e-6, decode, 0.32 -> 0.096; a box of them 21 -> 11
+// us; 336x272x208 f32 with chunks of 8, 0.14 -> 0.061 ms.
+template <uint32_t THREADS>
 struct UnpredShape {
     static constexpr uint32_t threads = THREADS;
-    static constexpr uint32_t tiles = TILES;                 // masks per thread
-    static constexpr uint32_t warp = 32 * 32 * TILES;        // codes a warp holds
-    static constexpr uint32_t span = warp * (THREADS / 32);  // codes the CTA holds
+    static constexpr uint32_t span = 32 * THREADS;  // codes the CTA holds
 };
-using UnpredBig = UnpredShape<1024, 1>;
-using UnpredLittle = UnpredShape<32, kUnpredSmall / 1024>;
+using UnpredBig = UnpredShape<1024>;
 template <class S>
 struct UnpredSmem {
     uint32_t wsum[S::threads / 32];
@@ -1256,7 +1253,7 @@ __device__ __forceinline__ void unpred_move_one(const UnpredWork& uw, const Stre
 {
     const StreamDesc s = sd[uw.stream];
     const uint32_t vol = s.C * s.C * s.C, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const bool alone = S::threads == 32 || vol <= S::warp;  // one warp's work
+    const bool alone = S::threads == 32 || vol <= 1024;  // one warp's work
     if (alone && wid) return;
     const uint32_t threads = alone ? 32u : S::threads;
     auto sync = [&]() {
@@ -1268,31 +1265,21 @@ __device__ __forceinline__ void unpred_move_one(const UnpredWork& uw, const Stre
     const bool vec = vol % 8 == 0 && ((uintptr_t)src & 15) == 0;
     uint64_t before = 0;  // zeros of the spans done
     for (uint32_t at = 0; at < vol && before < uw.count; at += S::span) {
-        const uint32_t w0 = wid * S::warp;  // from the span's start
-        uint32_t m[S::tiles], rank[S::tiles], n = 0;
+        const uint32_t i = at + threadIdx.x * 32;
+        uint32_t m = 0;
+        if (vec) {
 #pragma unroll
-        for (uint32_t t = 0; t < S::tiles; ++t) {
-            const uint32_t i = at + w0 + t * 1024 + lane * 32;
-            m[t] = 0;
-            if (vec) {
-#pragma unroll
-                for (uint32_t j = 0; j < 4; ++j)
-                    if (i + 8 * j < vol) {
-                        const uint4 q = __ldg(reinterpret_cast<const uint4*>(src + i + 8 * j));
-                        m[t] |= (pair_mask(q.x, 0) | pair_mask(q.y, 0) << 2 | pair_mask(q.z, 0) << 4 |
-                                 pair_mask(q.w, 0) << 6)
-                                << (8 * j);
-                    }
-            } else {
-                for (uint32_t j = 0; j < 32 && i + j < vol; ++j) m[t] |= (uint32_t)(src[i + j] == 0) << j;
-            }
+            for (uint32_t j = 0; j < 4; ++j)
+                if (i + 8 * j < vol) {
+                    const uint4 q = __ldg(reinterpret_cast<const uint4*>(src + i + 8 * j));
+                    m |= (pair_mask(q.x, 0) | pair_mask(q.y, 0) << 2 | pair_mask(q.z, 0) << 4 | pair_mask(q.w, 0) << 6)
+                         << (8 * j);
+                }
+        } else {
+            for (uint32_t j = 0; j < 32 && i + j < vol; ++j) m |= (uint32_t)(src[i + j] == 0) << j;
         }
-#pragma unroll
-        for (uint32_t t = 0; t < S::tiles; ++t) {
-            const uint32_t c = __popc(m[t]), incl = group_scan(c, 32, lane);
-            rank[t] = n + incl - c;
-            n += __shfl_sync(0xffffffffu, incl, 31);
-        }
+        const uint32_t c = __popc(m), incl = group_scan(c, 32, lane);
+        const uint32_t n = __shfl_sync(0xffffffffu, incl, 31);
         uint32_t r0 = 0, all = n;  // zeros before this warp's in the span, and in the span
         if (!alone) {
             if (lane == 0) sm.wsum[wid] = n;
@@ -1305,19 +1292,15 @@ __device__ __forceinline__ void unpred_move_one(const UnpredWork& uw, const Stre
                 all += v;
             }
         }
-#pragma unroll
-        for (uint32_t t = 0; t < S::tiles; ++t) {
-            uint32_t r = r0 + rank[t];
-            for (uint32_t mm = m[t]; mm; mm &= mm - 1, ++r)
-                sm.pos[r] = (uint16_t)(w0 + t * 1024 + lane * 32 + (__ffs(mm) - 1));
-        }
+        uint32_t r = r0 + incl - c;
+        for (uint32_t mm = m; mm; mm &= mm - 1, ++r) sm.pos[r] = (uint16_t)(threadIdx.x * 32 + (__ffs(mm) - 1));
         sync();
         for (uint32_t k = threadIdx.x; k < all; k += threads) {
-            const uint64_t r = before + k;
-            if (r >= uw.count) break;
+            const uint64_t v = before + k;
+            if (v >= uw.count) break;
             const size_t d = base + at + sm.pos[k];
-            if (GATHER) list[uw.list_off + r] = dense[d];
-            else dense[d] = list[uw.list_off + r];
+            if (GATHER) list[uw.list_off + v] = dense[d];
+            else dense[d] = list[uw.list_off + v];
         }
         sync();  // the list and wsum are written again
         before += all;
@@ -1436,18 +1419,18 @@ void unpred_move(bool gather, const UnpredWork* work, int nwork, const StreamDes
 }  // namespace
 
 template <typename T>
-void launch_unpred_move(bool gather, bool little, const UnpredWork* work, int nwork, const StreamDesc* sd,
+void launch_unpred_move(bool gather, uint32_t codes_most, const UnpredWork* work, int nwork, const StreamDesc* sd,
                         const uint16_t* codes, T* dense, T* list, cudaStream_t st)
 {
     if (!nwork) return;
-    if (little) unpred_move<UnpredLittle, T>(gather, work, nwork, sd, codes, dense, list, st);
+    if (codes_most <= 1024) unpred_move<UnpredShape<32>, T>(gather, work, nwork, sd, codes, dense, list, st);
+    else if (codes_most <= 4096) unpred_move<UnpredShape<128>, T>(gather, work, nwork, sd, codes, dense, list, st);
     else unpred_move<UnpredBig, T>(gather, work, nwork, sd, codes, dense, list, st);
 }
-uint32_t unpred_little_codes() { return kUnpredSmall; }
 
-template void launch_unpred_move<float>(bool, bool, const UnpredWork*, int, const StreamDesc*, const uint16_t*, float*,
+template void launch_unpred_move<float>(bool, uint32_t, const UnpredWork*, int, const StreamDesc*, const uint16_t*, float*,
                                         float*, cudaStream_t);
-template void launch_unpred_move<double>(bool, bool, const UnpredWork*, int, const StreamDesc*, const uint16_t*,
+template void launch_unpred_move<double>(bool, uint32_t, const UnpredWork*, int, const StreamDesc*, const uint16_t*,
                                          double*, double*, cudaStream_t);
 
 void launch_decode_dyn(int grid, const uint8_t* meta, const StreamDesc* sd, const uint16_t* cb_sym,

@@ -69,11 +69,10 @@ void launch_build_tables(const StreamDesc* sd, int nstreams, const uint16_t* cb_
 // group of small streams goes to the host in one transfer.
 void launch_pack_streams(const StreamDesc* sd, const uint64_t* stream_words, int s0, int s1, const uint32_t* payload,
                          uint32_t* dst, cudaStream_t st);
-// little: no listed chunk has more than unpred_little_codes() codes.
+// codes_most: the codes of the largest listed chunk.
 template <typename T>
-void launch_unpred_move(bool gather, bool little, const UnpredWork* work, int nwork, const StreamDesc* sd,
+void launch_unpred_move(bool gather, uint32_t codes_most, const UnpredWork* work, int nwork, const StreamDesc* sd,
                         const uint16_t* codes, T* dense, T* list, cudaStream_t st);
-uint32_t unpred_little_codes();
 
 // Persistent variants for captured graphs: `grid` CTAs walk the lists of a
 // batch held in device memory (BatchHdr at meta: n_work/o_work/o_ids,

@@ -205,15 +205,12 @@ template <typename T>
 stz_status level_error_bounds(stz_context* ctx, const T* field, size_t N, const stz_opts& o, int K, double& eb,
                               std::vector<double>& ebk);
 
-// No chunk of the listed unpredictable values is larger than
-// unpred_little_codes().
-inline bool unpred_little(const std::vector<StreamDesc>& sd, const UnpredWork* w, size_t n)
+// Codes of the largest chunk of the listed unpredictable values.
+inline uint32_t unpred_codes_most(const std::vector<StreamDesc>& sd, const UnpredWork* w, size_t n)
 {
-    for (size_t i = 0; i < n; ++i) {
-        const uint32_t C = sd[w[i].stream].C;
-        if (C * C * C > unpred_little_codes()) return false;
-    }
-    return true;
+    uint32_t C = 0;
+    for (size_t i = 0; i < n; ++i) C = std::max(C, sd[w[i].stream].C);
+    return C * C * C;
 }
 
 // CTA work items for chunk lists: groups of up to kCoderThreads / C chunks.

@@ -571,11 +571,12 @@ cudaError_t enqueue_bulk(SrvStream& ss, const uint8_t* hrec, const uint8_t* drec
         launch_decode(reinterpret_cast<const CtaWork*>(drec + h->o_work),
                       reinterpret_cast<const uint32_t*>(drec + h->o_ids), (int)h->n_work, p.d_sd, p.d_sym, p.d_tables,
                       p.d_sub, p.d_choff, p.d_payload, codes, st);
-    if (h->n_uwork)
-        launch_unpred_move<T>(
-            false, unpred_little(p.sd, reinterpret_cast<const UnpredWork*>(hrec + h->o_uwork), h->n_uwork),
-            reinterpret_cast<const UnpredWork*>(drec + h->o_uwork), (int)h->n_uwork, p.d_sd,
-                              codes, ss.unpred.as<T>(), (T*)p.d_ulist, st);
+    if (h->n_uwork) {
+        const uint32_t most =
+            unpred_codes_most(p.sd, reinterpret_cast<const UnpredWork*>(hrec + h->o_uwork), h->n_uwork);
+        launch_unpred_move<T>(false, most, reinterpret_cast<const UnpredWork*>(drec + h->o_uwork), (int)h->n_uwork,
+                              p.d_sd, codes, ss.unpred.as<T>(), (T*)p.d_ulist, st);
+    }
     for (const LevelJob& j : jobs) enqueue_level_job<T>(ss, j, st);
     return cudaGetLastError();
 }
