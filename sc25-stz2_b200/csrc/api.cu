@@ -192,6 +192,33 @@ void add_all_chunks(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint
     add_work(work, ids, stream, all.data(), all.size(), C);
 }
 
+// A chain of 1024 codes takes a thread about 0.18 ms, and lane groups take
+// about 1 us for each of a launch's items, 2 us where a warp's buffers do not
+// hold a plane (512^3 at the default chunks has 448 items in each half of its
+// finest level). k_decode on both sides of the lines: f32 GRF at 1e-3, 320^3,
+// 219 items, 0.23 by groups and 0.23 ms by plane, 384^3, 434 items, 0.33 and
+// 0.24; with chunks of 64, 256^3, 28 items, 0.39 and 0.86, 384^3, 94 items,
+// 1.31 and 0.70.
+constexpr size_t kPlaneItems = 256, kBigPlaneItems = 64;
+size_t plane_items(const std::vector<StreamDesc>& sd, std::vector<CtaWork>& work, size_t w0, size_t w1)
+{
+    size_t n = 0, big = 0;
+    for (size_t i = w0; i < w1; ++i) {
+        CtaWork& w = work[i];
+        const StreamDesc& d = sd[w.stream];
+        w.by_plane = d.run_n == 0 && d.C * d.C % 8 == 0 && d.code_off % 8 == 0 && w.count * d.C <= (uint32_t)kCoderThreads;
+        n += w.by_plane;
+        big += w.by_plane && d.C > 32;
+    }
+    if (n < kPlaneItems && big < kBigPlaneItems) {
+        for (size_t i = w0; i < w1; ++i) work[i].by_plane = 0;
+        return 0;
+    }
+    std::stable_partition(work.begin() + (ptrdiff_t)w0, work.begin() + (ptrdiff_t)w1,
+                          [](const CtaWork& w) { return w.by_plane != 0; });
+    return n;
+}
+
 int pool_threads(int requested)
 {
     if (requested > 0) return requested;
@@ -977,7 +1004,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
     uint64_t codes = 0, chunks = 0, subs = 0, words = 0, syms = 0, unp = 0;
     p.ulist_off.assign(nstreams + 1, 0);
     for (int i = 0; i < nstreams; ++i) {
-        const int k = i / 7 + 1;
+        const int k = i / 7 + 1, b = i % 7;
         const LevelDir& L = ps.lv[k];
         const StreamHeader& H = p.hdr[i];
         StreamDesc& d = p.sd[i];
@@ -985,6 +1012,7 @@ stz_status prepare(stz_context* ctx, const stz_stream* s, int kmax, Prepared& p,
         d.ncx = L.dx / L.C, d.ncy = L.dy / L.C, d.ncz = L.dz / L.C;
         d.nchunks = d.ncx * d.ncy * d.ncz;
         d.radius = h.radius;
+        if (b == 0) codes = (codes + 7) & ~(uint64_t)7;  // 16-byte groups of codes, where the level's size allows
         d.code_off = codes;
         codes += (uint64_t)L.dx * L.dy * L.dz;
         d.chunk_base = chunks;
@@ -1225,6 +1253,7 @@ struct DecodePipe {
     bool planned = false;
     size_t next_batch = 0;
     std::vector<size_t> wfirst, ufirst;  // per batch: first work / unpredictable item (+ end)
+    std::vector<size_t> nplanes;         // per batch: plane_items of its items
     std::vector<uint32_t> umost;         // per batch: unpred_codes_most of its items
     size_t o_w = 0, o_i = 0, o_u = 0;
     int next_level = 1, cur = 0;
@@ -1276,6 +1305,7 @@ struct DecodePipe {
             }
         }
         wfirst[batches.size()] = work.size();
+        for (size_t bi = 0; bi < batches.size(); ++bi) nplanes.push_back(plane_items(p.sd, work, wfirst[bi], wfirst[bi + 1]));
         ufirst[batches.size()] = uw.size();
         for (size_t bi = 0; bi < batches.size(); ++bi)
             umost.push_back(unpred_codes_most(p.sd, uw.data() + ufirst[bi], ufirst[bi + 1] - ufirst[bi]));
@@ -1339,9 +1369,15 @@ struct DecodePipe {
         if (copied) STZ_CUDA(cudaStreamWaitEvent(sd, copied, 0));
         const uint8_t* dw = ctx->work.as<uint8_t>();
         const size_t w0 = wfirst[bi], w1 = wfirst[bi + 1], u0 = ufirst[bi], u1 = ufirst[bi + 1];
-        if (w1 > w0) {
+        const size_t wp = w0 + nplanes[bi];
+        if (wp > w0) {
+            KScope ks(ctx, "k_decode_planes", 1, sd);
+            launch_decode_planes((const CtaWork*)(dw + o_w) + w0, (const uint32_t*)(dw + o_i), (int)(wp - w0), p.d_sd,
+                                 p.d_sym, p.d_tables, p.d_sub, p.d_choff, p.d_payload, ctx->codes.as<uint16_t>(), sd);
+        }
+        if (w1 > wp) {
             KScope ks(ctx, "k_decode", 1, sd);
-            launch_decode((const CtaWork*)(dw + o_w) + w0, (const uint32_t*)(dw + o_i), (int)(w1 - w0), p.d_sd,
+            launch_decode((const CtaWork*)(dw + o_w) + wp, (const uint32_t*)(dw + o_i), (int)(w1 - wp), p.d_sd,
                           p.d_sym, p.d_tables, p.d_sub, p.d_choff, p.d_payload, ctx->codes.as<uint16_t>(), sd);
         }
         if (u1 > u0) {
@@ -1546,6 +1582,7 @@ stz_status decompress_box_dev(stz_context* ctx, stz_stream* s, const int64_t lo[
         add_work(work, ids, si, cs.data(), cs.size(), high.C);
         add_unpred_work(*p, si, cs.data(), cs.size(), uw);
     }
+    const size_t nplanes = plane_items(p->sd, work, 0, work.size());
     lap.mark("work lists");
     // ROI jobs: the mid grid on the bounding box of the reference regions,
     // then the query box
@@ -1589,10 +1626,17 @@ stz_status decompress_box_dev(stz_context* ctx, stz_stream* s, const int64_t lo[
     const uint8_t* dm = ctx->work.as<uint8_t>();
     STZ_CUDA(ctx->codes.ensure(p->total_codes * 2));
     if (p->total_unpred) STZ_CUDA(ctx->unpred_dense.ensure(p->total_codes * sizeof(T)));
-    if (!work.empty()) {
+    if (nplanes) {
+        KScope ks(ctx, "k_decode_planes");
+        launch_decode_planes((const CtaWork*)(dm + hd.o_work), (const uint32_t*)(dm + hd.o_ids), (int)nplanes, p->d_sd,
+                             p->d_sym, p->d_tables, p->d_sub, p->d_choff, p->d_payload, ctx->codes.as<uint16_t>(),
+                             ctx->st);
+    }
+    if (work.size() > nplanes) {
         KScope ks(ctx, "k_decode");
-        launch_decode((const CtaWork*)(dm + hd.o_work), (const uint32_t*)(dm + hd.o_ids), (int)work.size(), p->d_sd,
-                      p->d_sym, p->d_tables, p->d_sub, p->d_choff, p->d_payload, ctx->codes.as<uint16_t>(), ctx->st);
+        launch_decode((const CtaWork*)(dm + hd.o_work) + nplanes, (const uint32_t*)(dm + hd.o_ids),
+                      (int)(work.size() - nplanes), p->d_sd, p->d_sym, p->d_tables, p->d_sub, p->d_choff, p->d_payload,
+                      ctx->codes.as<uint16_t>(), ctx->st);
     }
     if (!uw.empty()) {
         KScope ks(ctx, "k_unpred_move");

@@ -830,55 +830,50 @@ struct DecodeSmem {
     uint32_t max_len;
 };
 
-// Symbol decoding from a stream's tables, the lookup table itself in shared
-// or in global memory.
+// Symbol decoding from a stream's tables, those of each code in shared memory.
 struct DecodeCtx {
     const uint32_t* lut;
-    const uint4* len;  // where lut is
+    const uint4* len;
     uint32_t longest;
     const DecodeTables* __restrict__ t;
-    template <bool SMEM>
     __device__ __forceinline__ uint32_t entry(uint32_t bits) const
     {
-        return SMEM ? lut[bits >> (32 - kLutBits)] : __ldg(lut + (bits >> (32 - kLutBits)));
+        return lut[bits >> (32 - kLutBits)];
     }
     // The code at the top of bits: its length, and symbol or run length, or
     // canonical index (late).
-    template <bool SMEM>
     __device__ __forceinline__ void symbol(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
     {
-        const uint32_t e = entry<SMEM>(bits);
+        const uint32_t e = entry(bits);
         l = e & 31u, val = e >> 16, run = e & kLutRun, late = e & kLutLong;
         if (late) val = (bits >> (32 - l)) + val & 0xffffu;
-        if (l == 0) slow<SMEM>(bits, l, val, run, late);
+        if (l == 0) slow(bits, l, val, run, late);
     }
     // Its length, and how many codes it stands for.
-    template <bool SMEM>
     __device__ __forceinline__ void count(uint32_t bits, uint32_t& l, uint32_t& n) const
     {
-        const uint32_t e = entry<SMEM>(bits);
+        const uint32_t e = entry(bits);
         l = e & 31u, n = e & kLutRun ? e >> 16 : 1u;
         if (l == 0) {
             uint32_t val = e >> 16;
             bool run, late;
-            slow<SMEM>(bits, l, val, run, late);
+            slow(bits, l, val, run, late);
             n = run ? val : 1u;
         }
     }
     // val: the length to start from.
-    template <bool SMEM>
     __device__ __forceinline__ void slow(uint32_t bits, uint32_t& l, uint32_t& val, bool& run, bool& late) const
     {
         const uint32_t v = bits >> (32 - kMaxCodeLen);
         l = val;
-        while (l <= longest && v >= (SMEM ? len[l].x : __ldg(&len[l].x))) ++l;
+        while (l <= longest && v >= len[l].x) ++l;
         run = false, late = true;
         if (l > longest) {  // no code (corrupt stream): the codebook's first symbol, one bit
             l = 1;
             val = 0;
             return;
         }
-        const uint4 e = SMEM ? len[l] : __ldg(&len[l]);
+        const uint4 e = len[l];
         const uint32_t i = (bits >> (32 - l)) + e.y, r = i - e.z;
         run = r < (e.w & 0xffffu);
         val = run ? __ldg(&t->run[(e.w >> 16) + r]) : i;
@@ -896,7 +891,7 @@ __device__ __forceinline__ uint32_t peek(const Words& w, uint32_t pos)
 
 // Decode the plane of bits [r0, r1) by this lane's group of W lanes: the
 // literals go to put(code, value, late).
-template <bool SMEM, class Words, class Put>
+template <class Words, class Put>
 __device__ __forceinline__ void decode_plane(const DecodeCtx& dc, const Words& w, uint32_t r0, uint32_t r1, uint32_t W,
                                              uint32_t lane, Put&& put)
 {
@@ -907,7 +902,7 @@ __device__ __forceinline__ void decode_plane(const DecodeCtx& dc, const Words& w
         cnt = 0;
         while (end < stop) {
             uint32_t l, n;
-            dc.count<SMEM>(peek(w, end), l, n);
+            dc.count(peek(w, end), l, n);
             cnt += n;
             end += l;
         }
@@ -927,7 +922,7 @@ __device__ __forceinline__ void decode_plane(const DecodeCtx& dc, const Words& w
     while (start < stop) {
         uint32_t l, val;
         bool run, late;
-        dc.symbol<SMEM>(peek(w, start), l, val, run, late);
+        dc.symbol(peek(w, start), l, val, run, late);
         if (!run) put(q, val, late);
         q += run ? val : 1u;
         start += l;
@@ -985,40 +980,6 @@ __device__ __forceinline__ uint32_t fill_code(const StreamDesc& s, const uint16_
     return s.n_used == 1 && (uint32_t)syms[0] - s.run_base >= s.run_n ? (uint32_t)syms[0] : s.radius;
 }
 
-// Planes too large for the shared buffers: everything through L1, centre codes
-// stored first, literals over them.
-__device__ __forceinline__ void decode_direct(const StreamDesc& s, const DecodeTables* __restrict__ t, uint32_t W,
-                                              const uint32_t* __restrict__ chunks, uint32_t np, uint32_t first,
-                                              uint32_t nwarps, const uint16_t* __restrict__ cb_sym,
-                                              const uint32_t* __restrict__ sub_off,
-                                              const uint64_t* __restrict__ chunk_word_off,
-                                              const uint32_t* __restrict__ payload, uint16_t* __restrict__ codes)
-{
-    const uint32_t G = 32 / W, lane = threadIdx.x & (W - 1), gi = (threadIdx.x & 31) / W, P = s.C * s.C;
-    const uint16_t* __restrict__ syms = cb_sym + s.cb_off;
-    const uint32_t fill = fill_code(s, syms);
-    const bool by_index = t->by_index;
-    const DecodeCtx dc{t->lut, t->len, t->max_len, t};
-    for (uint32_t base = first * G; base < np; base += nwarps * G) {
-        const bool active = base + gi < np;
-        const PlaneAt a = plane_at(s, chunks, active ? base + gi : base, active, sub_off, chunk_word_off, payload, codes);
-        if (active) {
-            if (P % 8 == 0 && ((uintptr_t)a.dst & 15) == 0) {
-                const uint32_t f2 = fill * 0x10001u;
-                for (uint32_t k = lane; k < P / 8; k += W)
-                    reinterpret_cast<uint4*>(a.dst)[k] = make_uint4(f2, f2, f2, f2);
-            } else {
-                for (uint32_t k = lane; k < P; k += W) a.dst[k] = (uint16_t)fill;
-            }
-        }
-        __syncwarp();
-        decode_plane<false>(dc, [&](uint32_t i) { return __ldg(a.src + i); }, a.r0, a.r1, W, lane,
-                            [&](uint32_t q, uint32_t val, bool late) {
-                                if (q < P) a.dst[q] = late || by_index ? __ldg(syms + val) : (uint16_t)val;
-                            });
-    }
-}
-
 // Payload and table in shared memory, and the codes too where the warp's
 // planes fit its buffer: then only final values are stored, each once.
 __device__ __forceinline__ void decode_buffered(DecodeSmem& sm, const StreamDesc& s,
@@ -1067,9 +1028,12 @@ __device__ __forceinline__ void decode_buffered(DecodeSmem& sm, const StreamDesc
             }
         };
         const uint32_t nw = a.r1 > a.r0 ? ((a.r1 + 31) >> 5) + 2 : 0u;
+        const bool vec = P % 8 == 0 && ((uintptr_t)a.dst & 15) == 0;
         if (direct) {
-            if (active)
+            if (active && vec)
                 for (uint32_t k = lane; k < P / 8; k += W) reinterpret_cast<uint4*>(a.dst)[k] = f4;
+            else if (active)
+                for (uint32_t k = lane; k < P; k += W) a.dst[k] = (uint16_t)f2;
             __syncwarp();
         }
         if (__all_sync(0xffffffffu, nw <= cap)) {
@@ -1080,15 +1044,14 @@ __device__ __forceinline__ void decode_buffered(DecodeSmem& sm, const StreamDesc
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncwarp();
             const uint32_t* const sw = reinterpret_cast<const uint32_t*>(stage);
-            decode_plane<true>(dc, [&](uint32_t i) { return sw[i]; }, a.r0, a.r1, W, lane, put);
+            decode_plane(dc, [&](uint32_t i) { return sw[i]; }, a.r0, a.r1, W, lane, put);
         } else {
-            decode_plane<true>(dc, [&](uint32_t i) { return __ldg(a.src + i); }, a.r0, a.r1, W, lane, put);
+            decode_plane(dc, [&](uint32_t i) { return __ldg(a.src + i); }, a.r0, a.r1, W, lane, put);
         }
         __syncwarp();
         if (direct) continue;
         any_late = __any_sync(0xffffffffu, any_late);
         // the planes to global memory, the buffer back to its empty state
-        const bool vec = P % 8 == 0 && ((uintptr_t)a.dst & 15) == 0;
         for (uint32_t k = lane; k < Pc / 8; k += W) {
             const uint4 v = out[k];
             out[k] = f4;
@@ -1134,6 +1097,158 @@ __device__ __forceinline__ void load_table(DecodeSmem& sm, const DecodeTables* _
     __syncthreads();
 }
 
+// ---- decode: a thread per plane ---------------------------------------------------
+// In large launches a plane of a stream without run symbols is one thread's:
+// it decodes each code once, where a lane group decodes it about three times,
+// and the lanes of a warp write the same code of their planes in step. Bound by
+// the instructions of that step, with the plane's chain of codes as the least
+// time a launch takes, hence plane_items' rule on the number of items. The
+// table and the payload words lie in shared memory as above; the words are
+// fetched ahead by the same instruction for all lanes, since a load or a copy
+// that only some lanes issue makes the warp wait for it at the next one's use
+// (0.53 us a step with asynchronous copies per lane, 0.17 so). Where codes are
+// indexes, eight symbols are looked up together when they are stored.
+// k_decode, lane groups and now (levels below the finest and its two halves;
+// everything in one launch): 512^3 f32 GRF at 1e-2 0.74 -> 0.43; 0.65 -> 0.35
+// ms, at 1e-4 0.92 -> 0.70; 0.82 -> 0.57; 1024^3 at 1e-3 5.40 -> 2.65; 5.03 ->
+// 2.40. (A thread per plane through L1, as before the lane groups took all:
+// 0.98; 0.49, 1.18; 0.72, 3.63; 3.01.) Run symbols bring the lanes out of step:
+// fields with them took 0.58 -> 0.74 (512^3 f32 lognormal at 1e-4, one launch).
+constexpr int kPlaneThreads = kCoderThreads;
+constexpr uint32_t kRingWords = 32;  // payload words at hand of each thread
+struct PlaneSmem {
+    uint32_t lut[1 << kLutBits];
+    uint4 len[kMaxCodeLen + 1];
+    uint32_t ring[kRingWords][kPlaneThreads];
+    uint32_t max_len;
+};
+
+// A plane's bits in order. The words come through a ring in shared memory, two
+// 16-byte groups at a time, fetched and put into it by refill() every eight
+// symbols (which take six words at most): eleven words or more are always left.
+struct PlaneBits {
+    const uint4* __restrict__ src;
+    uint32_t (*ring)[kPlaneThreads];
+    uint32_t last;     // group that holds the word after the plane's last one
+    uint32_t fetched;  // groups in the ring so far
+    uint32_t wi;       // the word after next
+    uint64_t buf;      // the next bits on top, `have` >= 32 of them; next follows them
+    uint32_t next;
+    int have;
+    uint4 f0, f1;
+    bool flying;
+
+    __device__ __forceinline__ uint32_t word(uint32_t i) const { return ring[i % kRingWords][threadIdx.x]; }
+    __device__ __forceinline__ void put(uint32_t k, const uint4& v)
+    {
+        const uint32_t i = 4 * k % kRingWords, t = threadIdx.x;
+        ring[i][t] = v.x, ring[i + 1][t] = v.y, ring[i + 2][t] = v.z, ring[i + 3][t] = v.w;
+    }
+    __device__ __forceinline__ void init(const PlaneAt& a)
+    {
+        src = reinterpret_cast<const uint4*>(a.src);
+        last = (((a.r1 + 31) >> 5) + 1) >> 2;
+        fetched = kRingWords / 4 - 2;
+#pragma unroll
+        for (uint32_t k = 0; k < kRingWords / 4 - 2; ++k) put(k, __ldg(src + min(k, last)));
+        wi = a.r0 >> 5;
+        buf = ((uint64_t)word(wi) << 32 | word(wi + 1)) << (a.r0 & 31);
+        next = word(wi + 2);
+        wi += 3;
+        have = 64 - (int)(a.r0 & 31);
+        flying = false;
+    }
+    __device__ __forceinline__ void refill()
+    {
+        if (flying) {
+            put(fetched, f0), put(fetched + 1, f1);
+            fetched += 2;
+        }
+        flying = fetched <= last && fetched + 2 - (wi >> 2) <= kRingWords / 4;
+        if (flying) f0 = __ldg(src + fetched), f1 = __ldg(src + min(fetched + 1, last));
+    }
+    __device__ __forceinline__ uint32_t top() const { return (uint32_t)(buf >> 32); }
+    __device__ __forceinline__ void skip(uint32_t l)
+    {
+        buf <<= l;
+        have -= (int)l;
+        if (have < 32) {
+            buf |= (uint64_t)next << (32 - have);
+            have += 32;
+            next = word(wi++);
+        }
+    }
+};
+
+// The symbols of those of eight codes that are indexes (bit j of m: code j).
+__device__ __forceinline__ void look_up(uint32_t (&x)[4], uint32_t m, const uint16_t* __restrict__ syms)
+{
+    uint32_t y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (m >> j & 1u) y[j] = __ldg(syms + (x[j >> 1] >> (16 * (j & 1)) & 0xffffu));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (m >> j & 1u) x[j >> 1] = j & 1 ? (x[j >> 1] & 0xffffu) | y[j] << 16 : (x[j >> 1] & 0xffff0000u) | y[j];
+}
+
+// Planes of the listed chunks, a thread each; items of plane_items only.
+__global__ void __launch_bounds__(kPlaneThreads, 6)
+    k_decode_planes(const CtaWork* __restrict__ work, const uint32_t* __restrict__ chunk_ids,
+                    const StreamDesc* __restrict__ sd, const DecodeTables* __restrict__ tabs,
+                    const uint16_t* __restrict__ cb_sym, const uint32_t* __restrict__ sub_off,
+                    const uint64_t* __restrict__ chunk_word_off, const uint32_t* __restrict__ payload,
+                    uint16_t* __restrict__ codes)
+{
+    __shared__ __align__(16) PlaneSmem sm;
+    const CtaWork w = work[blockIdx.x];
+    const StreamDesc s = sd[w.stream];
+    const DecodeTables* __restrict__ t = tabs + w.stream;
+    {
+        const uint4* __restrict__ src = reinterpret_cast<const uint4*>(t->lut);
+        for (uint32_t i = threadIdx.x; i < (1u << kLutBits) / 4; i += kPlaneThreads)
+            reinterpret_cast<uint4*>(sm.lut)[i] = __ldg(src + i);
+        if (threadIdx.x <= kMaxCodeLen) sm.len[threadIdx.x] = __ldg(t->len + threadIdx.x);
+        if (threadIdx.x == 0) sm.max_len = t->max_len;
+    }
+    const uint16_t* __restrict__ syms = cb_sym + s.cb_off;
+    const uint32_t all = t->by_index ? 0xffu : 0u;
+    const uint32_t f2 = fill_code(s, syms) * 0x10001u;
+    const uint4 f4 = make_uint4(f2, f2, f2, f2);
+    __syncthreads();
+    const DecodeCtx dc{sm.lut, sm.len, sm.max_len, t};
+    const uint32_t P = s.C * s.C;
+    if (threadIdx.x >= w.count * s.C) return;
+    const PlaneAt a = plane_at(s, chunk_ids + w.first, threadIdx.x, true, sub_off, chunk_word_off, payload, codes);
+    uint4* const out = reinterpret_cast<uint4*>(a.dst);
+    if (a.r1 == a.r0) {  // a lone symbol has no bits
+        for (uint32_t g = 0; g < P / 8; ++g) out[g] = f4;
+        return;
+    }
+    PlaneBits b;
+    b.ring = sm.ring;
+    b.init(a);
+    for (uint32_t g = 0; g < P / 8; ++g) {
+        b.refill();
+        uint32_t x[4], m = all;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t top = b.top(), e = sm.lut[top >> (32 - kLutBits)];
+            uint32_t l = e & 31u, val = e >> 16;
+            if ((e & (kLutLong | 31u)) - 1u >= 31u) {  // no plain entry: an index
+                bool run, late;
+                if (l) val = (top >> (32 - l)) + val & 0xffffu;
+                else dc.slow(top, l, val, run, late);
+                m |= 1u << j;
+            }
+            b.skip(l);
+            x[j >> 1] = j & 1 ? x[j >> 1] | val << 16 : val;
+        }
+        if (m) look_up(x, m, syms);
+        out[g] = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+}
+
 // CTAs that share a work item: a plane per warp, down to a few per warp in
 // the largest launches. Short CTAs balance better than they pay for loading
 // the table (finest level's halves, 448 items, 512^3 f32 at 1e-4: 0.63 + 0.51
@@ -1170,11 +1285,6 @@ __global__ void __launch_bounds__(kDecodeThreads, LARGE ? 4 : 3)
         W = 16;
     if (blockIdx.y * kDecodeWarps * (32 / W) >= np) return;  // uniform per block
     const uint32_t first = blockIdx.y * kDecodeWarps + (threadIdx.x >> 5), nwarps = gridDim.y * kDecodeWarps;
-    if (P > kMaxPlane) {
-        decode_direct(s, tabs + w.stream, W, chunk_ids + w.first, np, first, nwarps, cb_sym, sub_off, chunk_word_off,
-                      payload, codes);
-        return;
-    }
     load_table(sm, tabs + w.stream);
     decode_buffered(sm, s, tabs + w.stream, W, chunk_ids + w.first, np, first, nwarps, cb_sym, sub_off, chunk_word_off,
                     payload, codes);
@@ -1206,11 +1316,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 3) k_decode_dyn(const uint8_t*
         const uint32_t P = s.C * s.C, W = decode_lanes(P), np = w.count * s.C;
         if (i % S * kDecodeWarps * (32 / W) >= np) continue;  // uniform per block
         const uint32_t first = i % S * kDecodeWarps + (threadIdx.x >> 5);
-        if (P > kMaxPlane) {
-            decode_direct(s, tabs + w.stream, W, chunk_ids + w.first, np, first, S * kDecodeWarps, cb_sym, sub_off,
-                          chunk_word_off, payload, codes);
-            continue;
-        }
         if (w.stream != loaded) load_table(sm, tabs + w.stream);
         loaded = w.stream;
         decode_buffered(sm, s, tabs + w.stream, W, chunk_ids + w.first, np, first, S * kDecodeWarps, cb_sym, sub_off,
@@ -1396,6 +1501,15 @@ void launch_decode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, co
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DecodeSmem));
     k<<<dim3(nwork, decode_slices((uint32_t)nwork)), kDecodeThreads, sizeof(DecodeSmem), st>>>(
         work, chunk_ids, sd, static_cast<const DecodeTables*>(tables), cb_sym, sub_off, chunk_word_off, payload, codes);
+}
+
+void launch_decode_planes(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
+                          const uint16_t* cb_sym, const void* tables, const uint32_t* sub_off,
+                          const uint64_t* chunk_word_off, const uint32_t* payload, uint16_t* codes, cudaStream_t st)
+{
+    if (nwork)
+        k_decode_planes<<<nwork, kPlaneThreads, 0, st>>>(work, chunk_ids, sd, static_cast<const DecodeTables*>(tables),
+                                                         cb_sym, sub_off, chunk_word_off, payload, codes);
 }
 
 size_t decode_tables_bytes() { return sizeof(DecodeTables); }

@@ -59,6 +59,10 @@ void launch_encode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, co
 void launch_decode(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
                    const uint16_t* cb_sym, const void* tables, const uint32_t* sub_off, const uint64_t* chunk_word_off,
                    const uint32_t* payload, uint16_t* codes, cudaStream_t st);
+// The same for items marked by_plane.
+void launch_decode_planes(const CtaWork* work, const uint32_t* chunk_ids, int nwork, const StreamDesc* sd,
+                          const uint16_t* cb_sym, const void* tables, const uint32_t* sub_off,
+                          const uint64_t* chunk_word_off, const uint32_t* payload, uint16_t* codes, cudaStream_t st);
 // Decode tables of every stream (read by the decoders): decode_tables_bytes()
 // each, stream i at byte i * decode_tables_bytes() of `tables`.
 size_t decode_tables_bytes();

@@ -213,6 +213,10 @@ inline uint32_t unpred_codes_most(const std::vector<StreamDesc>& sd, const Unpre
     return C * C * C;
 }
 
+// Moves the items of work[w0, w1) that decode a plane per thread
+// (k_decode_planes) to the front and marks them; returns how many there are.
+size_t plane_items(const std::vector<StreamDesc>& sd, std::vector<CtaWork>& work, size_t w0, size_t w1);
+
 // CTA work items for chunk lists: groups of up to kCoderThreads / C chunks.
 void add_work(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint32_t stream, const uint32_t* chunks,
               size_t n, int C);

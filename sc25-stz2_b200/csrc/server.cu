@@ -383,6 +383,7 @@ size_t pack(SrvStream& ss, Build& b, uint8_t* dst)
         add_work(b.work, b.ids, si, b.lists[j].data(), b.lists[j].size(), (int)ss.sd(si).C);
         add_unpred_work(*ss.p, si, b.lists[j].data(), b.lists[j].size(), b.uw);
     }
+    if (!b.jobs.empty()) plane_items(ss.p->sd, b.work, 0, b.work.size());  // (the fast lane's kernel takes any item)
     BatchHdr h{};
     h.n_work = (uint32_t)b.work.size();
     h.n_uwork = (uint32_t)b.uw.size();
@@ -567,10 +568,14 @@ cudaError_t enqueue_bulk(SrvStream& ss, const uint8_t* hrec, const uint8_t* drec
     const BatchHdr* h = reinterpret_cast<const BatchHdr*>(hrec);
     const Prepared& p = *ss.p;
     uint16_t* codes = ss.codes.as<uint16_t>();
-    if (h->n_work)
-        launch_decode(reinterpret_cast<const CtaWork*>(drec + h->o_work),
-                      reinterpret_cast<const uint32_t*>(drec + h->o_ids), (int)h->n_work, p.d_sd, p.d_sym, p.d_tables,
-                      p.d_sub, p.d_choff, p.d_payload, codes, st);
+    const CtaWork* hw = reinterpret_cast<const CtaWork*>(hrec + h->o_work);
+    const CtaWork* dw = reinterpret_cast<const CtaWork*>(drec + h->o_work);
+    const uint32_t* dids = reinterpret_cast<const uint32_t*>(drec + h->o_ids);
+    int np = 0;
+    while (np < (int)h->n_work && hw[np].by_plane) ++np;
+    launch_decode_planes(dw, dids, np, p.d_sd, p.d_sym, p.d_tables, p.d_sub, p.d_choff, p.d_payload, codes, st);
+    launch_decode(dw + np, dids, (int)h->n_work - np, p.d_sd, p.d_sym, p.d_tables, p.d_sub, p.d_choff, p.d_payload, codes,
+                  st);
     if (h->n_uwork) {
         const uint32_t most =
             unpred_codes_most(p.sd, reinterpret_cast<const UnpredWork*>(hrec + h->o_uwork), h->n_uwork);

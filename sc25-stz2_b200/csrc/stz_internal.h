@@ -175,7 +175,7 @@ struct CtaWork {
     uint32_t stream;
     uint32_t first;
     uint32_t count;
-    uint32_t pad;
+    uint32_t by_plane;  // decode: a plane per thread (plane_items)
 };
 
 // Header of a request batch in device memory (request server). The arrays
