@@ -192,25 +192,31 @@ void add_all_chunks(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint
     add_work(work, ids, stream, all.data(), all.size(), C);
 }
 
-// A chain of 1024 codes takes a thread about 0.18 ms, and lane groups take
-// about 1 us for each of a launch's items, 2 us where a warp's buffers do not
-// hold a plane (512^3 at the default chunks has 448 items in each half of its
-// finest level). k_decode on both sides of the lines: f32 GRF at 1e-3, 320^3,
-// 219 items, 0.23 by groups and 0.23 ms by plane, 384^3, 434 items, 0.33 and
-// 0.24; with chunks of 64, 256^3, 28 items, 0.39 and 0.86, 384^3, 94 items,
-// 1.31 and 0.70.
-constexpr size_t kPlaneItems = 256, kBigPlaneItems = 64;
+// A chain of P codes takes a thread about 0.18 P / 1024 ms, and lane groups take
+// about 1 us for 128 planes of 1024 codes, 2.5 us for each 1024 codes of theirs
+// where a warp's buffers do not hold a plane. The line lies at 256 items of 128
+// planes, 64 of larger planes; planes smaller than the launch's largest count
+// for what they are of it (a box of 256^3 in a 512^3 field has 330 items, 110
+// of them of 256 codes a plane: 0.41 ms by groups, 0.43 by plane). k_decode on
+// both sides: f32 GRF at 1e-3, 320^3, 219 items, 0.23 by groups and 0.23 ms by
+// plane, 384^3, 434 items, 0.33 and 0.24; with chunks of 64, 256^3, 28 items,
+// 0.39 and 0.86, 384^3, 94 items, 1.31 and 0.70.
+constexpr uint64_t kPlaneItems = 256, kBigPlaneItems = 64;
 size_t plane_items(const std::vector<StreamDesc>& sd, std::vector<CtaWork>& work, size_t w0, size_t w1)
 {
-    size_t n = 0, big = 0;
+    size_t n = 0;
+    uint64_t codes = 0, most = 0;  // of the items that could, and of their largest plane
     for (size_t i = w0; i < w1; ++i) {
         CtaWork& w = work[i];
         const StreamDesc& d = sd[w.stream];
-        w.by_plane = d.run_n == 0 && d.C * d.C % 8 == 0 && d.code_off % 8 == 0 && w.count * d.C <= (uint32_t)kCoderThreads;
-        n += w.by_plane;
-        big += w.by_plane && d.C > 32;
+        const uint64_t P = (uint64_t)d.C * d.C;
+        w.by_plane = d.run_n == 0 && P % 8 == 0 && d.code_off % 8 == 0 && w.count * d.C <= (uint32_t)kCoderThreads;
+        if (!w.by_plane) continue;
+        ++n;
+        codes += w.count * d.C * P;
+        most = std::max(most, P);
     }
-    if (n < kPlaneItems && big < kBigPlaneItems) {
+    if (codes < (most > 1024 ? kBigPlaneItems : kPlaneItems) * kCoderThreads * std::max<uint64_t>(most, 1)) {
         for (size_t i = w0; i < w1; ++i) work[i].by_plane = 0;
         return 0;
     }

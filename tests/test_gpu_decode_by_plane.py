@@ -1,6 +1,6 @@
 """The decoder that gives every plane a thread: whole decodes of resident
 streams and large boxes equal to the oracle's where its launches are large
-enough (256 work items, 64 of planes past 1024 codes) and below, for plane sizes
+enough (256 items of 128 planes, 64 of planes past 1024 codes) and below, for plane sizes
 that are multiples of 8, for plane counts that leave its last threads idle, for
 codes of every length (a few symbols, long codes, every code value, 24 bits), for lone
 symbols, for streams with run symbols or planes of odd sizes among the others,
@@ -106,7 +106,7 @@ def test_served_levels_by_plane(ctx):
     from stz_b200 import Server
 
     dims = (144, 144, 144)
-    f = _field(["rough", "runs"], dims, np.float32, np.random.default_rng(1))
+    f = _field(["rough", "rough", "runs"], dims, np.float32, np.random.default_rng(1))
     f[::3, 1::2, ::5] += 1e6  # a list of unpredictable values
     want = po.compress(f, 0.5, chunk_high=8, chunk_low=4, mults=(1.0, 1.0, 1.0))
     full = po.decompress(want)
