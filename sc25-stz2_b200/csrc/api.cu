@@ -201,16 +201,23 @@ void add_all_chunks(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint
 // both sides: f32 GRF at 1e-3, 320^3, 219 items, 0.23 by groups and 0.23 ms by
 // plane, 384^3, 434 items, 0.33 and 0.24; with chunks of 64, 256^3, 28 items,
 // 0.39 and 0.86, 384^3, 94 items, 1.31 and 0.70.
+// STZ_DECODE_SEQ_BITS keeps streams below that many payload bits a plane on
+// average with the lane groups (0, the default: none), for comparisons.
 constexpr uint64_t kPlaneItems = 256, kBigPlaneItems = 64;
 size_t plane_items(const std::vector<StreamDesc>& sd, std::vector<CtaWork>& work, size_t w0, size_t w1)
 {
+    static const uint64_t seq_bits = [] {
+        const char* e = std::getenv("STZ_DECODE_SEQ_BITS");
+        return e ? (uint64_t)std::strtoull(e, nullptr, 10) : 0;
+    }();
     size_t n = 0;
     uint64_t codes = 0, most = 0;  // of the items that could, and of their largest plane
     for (size_t i = w0; i < w1; ++i) {
         CtaWork& w = work[i];
         const StreamDesc& d = sd[w.stream];
         const uint64_t P = (uint64_t)d.C * d.C;
-        w.by_plane = d.run_n == 0 && P % 8 == 0 && d.code_off % 8 == 0 && w.count * d.C <= (uint32_t)kCoderThreads;
+        w.by_plane = d.run_n == 0 && P % 8 == 0 && d.code_off % 8 == 0 && w.count * d.C <= (uint32_t)kCoderThreads &&
+                     32 * (d.word_cap - 4) >= seq_bits * d.nchunks * d.C;
         if (!w.by_plane) continue;
         ++n;
         codes += w.count * d.C * P;

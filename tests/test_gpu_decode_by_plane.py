@@ -6,10 +6,16 @@ codes of every length (a few symbols, long codes, every code value, 24 bits), fo
 symbols, for streams with run symbols or planes of odd sizes among the others,
 and served. Codes are chosen as in test_gpu_codebook: a zero coarse grid,
 multipliers 1, eb 0.5."""
+import hashlib
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import pyoracle as po
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +129,36 @@ def test_served_levels_by_plane(ctx):
             srv.release(x)
     finally:
         srv.close()
+
+
+CHILD = r"""
+import hashlib, sys
+sys.path[:0] = sys.argv[1:3]
+import numpy as np
+import stz_b200
+ctx = stz_b200.Context(0)
+s = ctx.parse(open(sys.argv[3], "rb").read())
+ctx.upload(s)
+ctx.profile_reset()
+out = ctx.decompress(s)
+print(ctx.profile_read().get("k_decode_planes", (0, 0))[1], hashlib.sha256(out.tobytes()).hexdigest())
+"""
+
+
+@pytest.mark.parametrize("bits,by_plane", [(None, True), ("0", True), ("200", True), ("1000", False), ("4294967295", False)])
+def test_the_switch_between_the_two_forms(tmp_path, bits, by_plane):
+    """STZ_DECODE_SEQ_BITS, read once a process: the least payload bits a plane
+    (64 codes of about 10 bits here) for a thread per plane. Same output."""
+    dims = (144, 144, 144)
+    f = _field(["rough"], dims, np.float32, np.random.default_rng(2))
+    want = po.compress(f, 0.5, chunk_high=8, chunk_low=4, mults=(1.0, 1.0, 1.0))
+    (tmp_path / "s").write_bytes(want)
+    env = {k: v for k, v in os.environ.items() if k != "STZ_DECODE_SEQ_BITS"}
+    if bits is not None:
+        env["STZ_DECODE_SEQ_BITS"] = bits
+    r = subprocess.run([sys.executable, "-c", CHILD, os.path.join(ROOT, "sc25-stz2_b200"), ROOT, str(tmp_path / "s")],
+                       capture_output=True, text=True, env=env, timeout=300)
+    assert r.returncode == 0, r.stderr
+    n, h = r.stdout.split()[-2:]
+    assert (int(n) > 0) == by_plane
+    assert h == hashlib.sha256(po.decompress(want).tobytes()).hexdigest()
