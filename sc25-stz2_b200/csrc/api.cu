@@ -195,12 +195,15 @@ void add_all_chunks(std::vector<CtaWork>& work, std::vector<uint32_t>& ids, uint
 // A chain of P codes takes a thread about 0.18 P / 1024 ms, and lane groups take
 // about 1 us for 128 planes of 1024 codes, 2.5 us for each 1024 codes of theirs
 // where a warp's buffers do not hold a plane. The line lies at 256 items of 128
-// planes, 64 of larger planes; planes smaller than the launch's largest count
+// planes, 64 of larger planes. Planes smaller than the launch's largest count
 // for what they are of it (a box of 256^3 in a 512^3 field has 330 items, 110
-// of them of 256 codes a plane: 0.41 ms by groups, 0.43 by plane). k_decode on
-// both sides: f32 GRF at 1e-3, 320^3, 219 items, 0.23 by groups and 0.23 ms by
-// plane, 384^3, 434 items, 0.33 and 0.24; with chunks of 64, 256^3, 28 items,
-// 0.39 and 0.86, 384^3, 94 items, 1.31 and 0.70.
+// of them of 256 codes a plane: 0.41 ms by groups, 0.43 by plane), and streams
+// of more than 12 bits a code for half: most of their codes are looked up in the
+// codebook, which a thread waits for. k_decode of whole fields on both sides, by
+// groups and by plane: f32 GRF at 1e-3, 320^3, 250 items so counted, 0.23 and
+// 0.23 ms, 384^3, 430 items, 0.33 and 0.24; with chunks of 64, 256^3, 56 items,
+// 0.39 and 0.86, 384^3, 110 items, 1.31 and 0.70; at 1e-5 (13.3 bits), 384^3,
+// 215 items, 0.47 and 0.54, 512^3, 510 items, 1.08 and 1.00.
 // STZ_DECODE_SEQ_BITS keeps streams below that many payload bits a plane on
 // average with the lane groups (0, the default: none), for comparisons.
 constexpr uint64_t kPlaneItems = 256, kBigPlaneItems = 64;
@@ -220,7 +223,8 @@ size_t plane_items(const std::vector<StreamDesc>& sd, std::vector<CtaWork>& work
                      32 * (d.word_cap - 4) >= seq_bits * d.nchunks * d.C;
         if (!w.by_plane) continue;
         ++n;
-        codes += w.count * d.C * P;
+        const bool wide = 32 * (d.word_cap - 4) > 12 * P * d.C * d.nchunks;
+        codes += w.count * d.C * P / (wide ? 2 : 1);
         most = std::max(most, P);
     }
     if (codes < (most > 1024 ? kBigPlaneItems : kPlaneItems) * kCoderThreads * std::max<uint64_t>(most, 1)) {

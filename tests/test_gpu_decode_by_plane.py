@@ -60,7 +60,8 @@ def _launches(ctx, fn):
 CASES = [
     (["rough"], (144, 144, 144), 8, True),       # 7 x 46 items, the last of each 9 chunks of 16
     (["narrow"], (144, 144, 144), 8, True),
-    (["widest"], (144, 144, 144), 8, True),
+    (["widest"], (144, 144, 144), 8, False),     # 16 bits a code: count for half
+    (["widest"], (176, 176, 176), 8, True),
     (["longest"], (160, 144, 144), 8, True),
     (["lone"], (144, 144, 144), 8, True),        # no bits at all
     (["rough", "runs", "lone"], (200, 200, 200), 10, False),  # planes of 100 codes: not a multiple of 8
