@@ -138,7 +138,17 @@ const char* stz_status_string(stz_status s);
 const char* stz_last_error(void);
 
 /* Context: one CUDA device, one CUDA stream, cached device/pinned buffers and
- * a host thread pool for zstd. */
+ * a host thread pool for zstd. Its buffers grow to what its largest calls need
+ * and are given back when it is destroyed. Besides the field-sized ones, a
+ * context that has compressed keeps 62 bytes of device memory per code value
+ * (2 * radius) and stream for the codebooks' scratch and 7 for the code tables
+ * and lists (about 95 MB at the default radius with three levels of 64^3 and
+ * more codes a block; smaller levels take the bytes per code of theirs), and
+ * on the host the frames and headers of a call (at most 1 GiB). One that has
+ * decompressed streams that are not resident keeps the parsed headers of the
+ * last one, and pageable host arrays move through two pinned chunks of at most
+ * 32 MiB. Freed streams' memory is kept for the next ones, at most four blocks
+ * and 2 GiB in the process. */
 stz_status stz_context_create(int device, stz_context** out);
 void stz_context_destroy(stz_context* ctx);
 /* Wait for all work queued on the context's stream. */

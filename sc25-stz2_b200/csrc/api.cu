@@ -529,11 +529,11 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
                     KScope ks(ctx, "k_learned_eval");
                     launch_learned_eval<T>(a, ctx->eval.as<uint32_t>(), st);
                 }
-                STZ_CUDA(ctx->h_hist.ensure(2 * 7 * kEvalBins * 4));
-                STZ_CUDA(cudaMemcpyAsync(ctx->h_hist.p, ctx->eval.p, 2 * 7 * kEvalBins * 4, cudaMemcpyDeviceToHost,
+                STZ_CUDA(ctx->h_books.ensure(2 * 7 * kEvalBins * 4));
+                STZ_CUDA(cudaMemcpyAsync(ctx->h_books.p, ctx->eval.p, 2 * 7 * kEvalBins * 4, cudaMemcpyDeviceToHost,
                                          st));
                 STZ_CUDA(cudaStreamSynchronize(st));
-                lflags[k] = choose_learned_flags(ctx->h_hist.as<uint32_t>(), elem);
+                lflags[k] = choose_learned_flags(ctx->h_books.as<uint32_t>(), elem);
             }
             a.learned.flags = lflags[k];
             if (!lflags[k]) a.learned.model = nullptr, a.learned.flags = 0;
@@ -710,8 +710,8 @@ stz_status compress_impl(stz_context* ctx, const T* field, int nx, int ny, int n
     STZ_CUDA(cudaStreamWaitEvent(sc, named[EvLevels], 0));
     STZ_CUDA(cudaMemcpyAsync(h_ucnt, ctx->unpred_cnt.p, g.total_chunk_slots * 4, cudaMemcpyDeviceToHost, sc));
     STZ_CUDA(cudaEventRecord(named[EvCounts], sc));
-    STZ_CUDA(ctx->h_hist.ensure(o_len + cb_cap));
-    uint8_t* hb = ctx->h_hist.as<uint8_t>();
+    STZ_CUDA(ctx->h_books.ensure(o_len + cb_cap));
+    uint8_t* hb = ctx->h_books.as<uint8_t>();
     STZ_CUDA(cudaStreamWaitEvent(sc, named[EvBooks], 0));
     STZ_CUDA(cudaMemcpyAsync(hb, dbooks, (size_t)nstreams * sizeof(CodebookInfo), cudaMemcpyDeviceToHost, sc));
     STZ_CUDA(cudaEventRecord(named[EvInfo], sc));

@@ -15,7 +15,7 @@
 // code tables (one B200, 16 host cores), host before and both kernels here
 // now: 64^3 f32 0.52 -> 0.058 ms, 512^3 f32 at rel 1e-3 0.25 -> 0.073 ms and
 // at 1e-4 1.4 -> 0.11 ms, 384x384x256 f64 fronts at 1e-6 (codebooks of up to
-// 60 K symbols) 12-14 -> 0.69 ms, 1.07 ms of it before the searches of a
+// 65 K symbols) 12-14 -> 0.69 ms, 1.07 ms of it before the searches of a
 // thread ran four side by side and the sort loaded four items ahead. The
 // merges of up to kSmallBook symbols are one warp's work in shared memory:
 // 0.085 -> 0.073 ms on the 512^3 field at 1e-3.

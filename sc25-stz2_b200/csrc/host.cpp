@@ -356,7 +356,7 @@ void* pooled_alloc(size_t bytes)
         }
     }
     size_t step = kPoolMin;
-    while (16 * step <= bytes) step *= 2;  // an eighth to a sixteenth of the size
+    while (16 * step <= bytes) step *= 2;  // from 8 MiB on at most an eighth of the size
     const size_t cap = (bytes + step - 1) / step * step;
     void* blk = std::malloc(cap + kPoolHdr);
     if (!blk) return nullptr;

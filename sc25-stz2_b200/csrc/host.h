@@ -26,8 +26,9 @@ namespace stz {
 // Large byte blocks come from a small process-wide pool of recently freed
 // blocks (their pages stay mapped, so writing a new container does not fault
 // and zero fresh pages); the pool keeps at most 4 blocks and 2 GiB. Blocks are
-// rounded up by at most an eighth, so that the next stream of about the same
-// size fits a freed one, and large ones ask for huge pages.
+// rounded up to whole MiB, larger ones by at most an eighth, so that the next
+// stream of about the same size fits a freed one, and large ones ask for huge
+// pages.
 void* pooled_alloc(size_t bytes);
 void pooled_free(void* p, size_t bytes);
 

@@ -12,8 +12,9 @@
 // "sub-chunk") has its bit offset inside the chunk in the stream header, so
 // all planes of all chunks of all streams encode and decode independently.
 // Inside a plane, the encode side shares the codes among a group of lanes
-// (runs are the gaps between literal masks); the decoder gives a lane to each
-// plane. Bits are packed MSB-first into 32-bit words; a chunk starts on a
+// (runs are the gaps between literal masks); the decode side shares the bits
+// among one, or, in large launches of streams without runs, gives a plane a
+// thread. Bits are packed MSB-first into 32-bit words; a chunk starts on a
 // word boundary.
 //
 // Runs: inside a plane, a maximal run of r centre codes (code == radius) is
@@ -687,23 +688,23 @@ __global__ void __launch_bounds__(kLaneThreads) k_encode(const CtaWork* __restri
 //     indexes only.
 // Before, table, payload words and symbols were read through L1 in the chain,
 // the length of a long code was searched there, and dense streams of large
-// launches had one thread per plane, whose lanes diverged. Launch times on one
+// launches had one thread per plane (below, in today's form). Launch times on one
 // B200, then and now (levels below the finest and its two halves together):
 //   512^3 f32 at 1e-3          0.430 -> 0.338 ms
 //   512^3 f32 at 1e-4          1.968 -> 0.687 ms
-//   384x384x256 f64 at 1e-6    1.310 -> 0.464 ms
+//   384x384x256 f64 at 1e-6    1.310 -> 0.464 ms (its halves stay below plane_items' line)
 //   its boxes of 16-128 a side 0.156 -> 0.048 ms a box
 // (With one step function for counting and placing, the search from kLutBits
 // up and through L1, and one build for launches of all sizes: 0.41, 0.86, 0.56
 // and 0.068 ms.)
-// Tried as well: one lane per plane in lockstep (windows of codes in shared
-// memory, payload rings filled by asynchronous copies), 0.17 / 0.62 / 0.42 ms
-// at 1e-4 and a chain of 1024 symbols in every small launch; several symbols
+// Tried as well: one lane per plane in lockstep for all streams (windows of
+// codes in shared memory, payload rings filled by asynchronous copies), 0.17 /
+// 0.62 / 0.42 ms at 1e-4 and a chain of 1024 symbols in every small launch; several symbols
 // per lookup in the counting passes (fewer instructions, more table to load:
 // even); four lanes' worth of planes per warp for all streams (fewer warps
 // resident: slower); only the planes that a box needs, as work items of equal
-// plane ranges (a box's decode is the chain of two or three planes in each
-// warp, and chunks with unpredictable values start at plane 0: even).
+// plane ranges (a box's decode is the chain of the one plane that each of its
+// warps has, which fewer planes do not shorten: even).
 
 // lut entry: code length in bits 0-4 (0: the prefix spans lengths, holds long
 // run symbols, or no code; bits 16-31 then hold the shortest length above

@@ -209,12 +209,12 @@ constexpr int kSmemBins = 448;
 
 struct HistArgs {
     uint32_t* full;     // 7 x 2r bins
-    uint32_t* outside;  // 7 flags: the stream has codes outside the window (kHistWindow)
+    uint32_t* outside;  // 7 flags: the stream has codes more than kHistWindow / 2 from the centre
     int radius;
 };
 
 // A thread's counter of one stream's centre codes also holds a flag: it had a
-// code outside the window. As an atomic counter per stream, every code of a
+// code that far from the centre. As an atomic counter per stream, every code of a
 // wide stream went to the same seven words, and one L2 slice held the kernel
 // up (93 % of that slice's tag lookups, 20 % over all; finest level of
 // 384x384x256 f64 at 1e-6: 0.718 -> 0.337 ms, of 512^3 f32 0.407 -> 0.396).
@@ -253,7 +253,7 @@ __device__ __forceinline__ void hist_code(uint32_t (*sh)[kSmemBins], int wlo, in
 }
 
 // Flush the per-thread dominant-bin counters (warp sum, one atomic per warp)
-// and the flags of codes outside the window (one store per warp and stream).
+// and the flags of codes far from the centre (one store per warp and stream).
 __device__ __forceinline__ void hist_flush_center(uint32_t (*sh)[kSmemBins], int wlo, int wn, const HistArgs& h,
                                                   const uint32_t (&center)[7])
 {

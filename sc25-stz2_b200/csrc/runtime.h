@@ -295,13 +295,13 @@ struct stz_context {
     stz::DevBuf field, grid[2], codes, unpred_dense, unpred_cnt, hist, hist_out, ctab, sub_bits, sub_off, chunk_off,
         stream_words, payload, sd, work, ids, uwork, ulist, books, cb_scratch, minmax, packed, rbits, out, mid, boxes,
         tiles, models, eval, rstats, staged_full;
-    stz::PinBuf h_hist, h_meta, h_meta2, h_payload, h_stage, h_io, h_small;
+    stz::PinBuf h_books, h_meta, h_meta2, h_payload, h_stage, h_io, h_small;
     size_t io_read = 0, payload_read = 0;  // bytes of h_io and h_payload that the host read in the last compress
     stz::PinBuf h_xfer[2];  // staging chunks of host <-> device copies of pageable caller buffers
     // device buffers lent to one-off decodes
     stz::DevBuf p_stage, p_coarsest, p_base;
-    // host memory kept between calls: frames and headers of a call, and the
-    // parsed headers of one-off decodes
+    // host memory kept between calls until the context goes: frames and headers
+    // of a call (at most 1 GiB), and the parsed headers of one-off decodes
     stz::HostArena arena;
     std::vector<stz::StreamHeader> hdr_scratch;
     void borrow(stz::Prepared& p)

@@ -15,8 +15,9 @@ void set_last_error(const std::string& msg);
 constexpr int kMaxCodeLen = 24;
 // Fast decode table width (bits) of the GPU decoder.
 constexpr int kLutBits = 12;
-// Codes around the radius that a codebook looks at when a stream has no others
-// (the encoder flags the streams that do; they have every code looked at).
+// Codes [radius - kHistWindow / 2, radius + kHistWindow / 2) are all that a
+// codebook looks at in a stream without others (the level encoders flag the
+// streams that have some; those have every code looked at).
 constexpr int kHistWindow = 4096;
 // Planes of one coder work item: an item covers max(1, 128 / C) chunks of a
 // stream, i.e. up to 128 planes (the coder kernels split an item over
